@@ -102,9 +102,10 @@ typedef struct {
  * (warps claim rays in chunks from a per-stream device counter and refill
  * finished lanes). */
 #define ILM_FLAG_GRID_SCHEDULE 2
-/* Persistent schedule compiled for many resident blocks per SM instead of
- * the compiler's register choice: 7 (up to 72 registers per thread) for the
- * pooled kernel, 8 (64) for the lane-refill kernel. */
+/* Persistent schedule compiled for many resident blocks per SM (7 for the
+ * wide layouts, up to 72 registers per thread; 8 for kd-trees, 64) instead of
+ * the compiler's register choice.  Accels of triangles alone run that build
+ * with or without the flag; it decides for accels with quadrics or curves. */
 #define ILM_FLAG_HIGH_OCCUPANCY 4
 /* Persistent schedule: each idle lane tests its own claimed rays against the
  * scene's root box instead of the whole warp testing each claimed chunk and

@@ -160,7 +160,7 @@ inline LaunchParams accel_launch(const ilm_context* ctx, const Accel* a) {
     const int persistent = a->schedule >= 0 ? (a->schedule == 0) : !(ctx->flags & ILM_FLAG_GRID_SCHEDULE);
     const int high_occ = a->high_occupancy >= 0 ? a->high_occupancy : (ctx->flags & ILM_FLAG_HIGH_OCCUPANCY) != 0;
     LaunchParams lp{a->stack_depth > 0 ? a->stack_depth : ctx->stack_depth, ctx->block_size, ctx->max_iter,
-                    persistent, nullptr, high_occ ? 8 : 0, (ctx->flags & ILM_FLAG_LANE_REFILL) ? 0 : 1};
+                    persistent, nullptr, high_occ, (ctx->flags & ILM_FLAG_LANE_REFILL) ? 0 : 1};
     lp.split_tail = split_tail_of(ctx);
     return lp;
 }

@@ -26,7 +26,8 @@ struct LaunchParams {
     uint32_t max_iter;         // per-ray loop cap
     int persistent;            // wide layouts: persistent schedule (needs `counter`)
     unsigned long long* counter;   // device work counter, private to the launch's stream
-    int min_blocks;            // persistent kernel occupancy hint (8 = 64-register variant)
+    int high_occupancy;        // persistent kernels with analytic shapes: the build for many resident
+                               // blocks per SM (accels of triangles alone always run it)
     int root_pool;             // persistent schedule: claimed chunks tested against the root box by the
                                // whole warp, entering rays pooled per warp (1), or each idle lane
                                // testing its own claims (0)

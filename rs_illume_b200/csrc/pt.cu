@@ -710,7 +710,7 @@ int32_t setup_render(ilm_context* ctx, PtScene& sc, uint32_t spp, uint32_t max_d
     unsigned long long* counter = ctx->counter_for(r.s);
     if (!counter) return ILM_ERR_OUT_OF_MEMORY;
     r.lp = LaunchParams{ctx->stack_depth, ctx->block_size, ctx->max_iter, 1, counter,
-                        (ctx->flags & ILM_FLAG_HIGH_OCCUPANCY) ? 8 : 0,
+                        (ctx->flags & ILM_FLAG_HIGH_OCCUPANCY) != 0,
                         1};   // pooled refill with the split tail (2,484-2,491 against 2,451
                               // Mrays/s for lanes that refill one by one, at 7 blocks per SM)
     // Queues of at most one wave (late bounces, training suffixes) run one

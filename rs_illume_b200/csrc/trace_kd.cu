@@ -345,11 +345,17 @@ cudaError_t launch_persistent(const TraceArgs& t, cudaStream_t s) {
 template <bool kAnalytic>
 cudaError_t launch_kd(const TraceArgs& t, const LaunchParams& lp, cudaStream_t s) {
     if (lp.persistent && t.counter) {
-        if (lp.root_pool)
-            return lp.min_blocks >= 8 ? launch_persistent<8, kAnalytic, true>(t, s)
-                                      : launch_persistent<1, kAnalytic, true>(t, s);
-        return lp.min_blocks >= 8 ? launch_persistent<8, kAnalytic, false>(t, s)
-                                  : launch_persistent<1, kAnalytic, false>(t, s);
+        // Trees of triangles alone always run the build for 8 resident blocks
+        // per SM (62 registers, no spills): 500,001 ball rays on 327,680
+        // triangles 414 against 436 us with the compiler's own
+        // register choice.  With analytic shapes the caller's flag decides.
+        if constexpr (kAnalytic) {
+            if (!lp.high_occupancy)
+                return lp.root_pool ? launch_persistent<1, kAnalytic, true>(t, s)
+                                    : launch_persistent<1, kAnalytic, false>(t, s);
+        }
+        return lp.root_pool ? launch_persistent<8, kAnalytic, true>(t, s)
+                            : launch_persistent<8, kAnalytic, false>(t, s);
     }
     const unsigned block = kKdBlock;
     unsigned grid = (unsigned)((t.n + block - 1) / block);

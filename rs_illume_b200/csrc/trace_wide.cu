@@ -91,8 +91,7 @@ __global__ void __launch_bounds__(128) k_trace_wide_split(TraceArgs a) {
 }
 
 // kMinBlocks > 0 asks the compiler for that many resident 128-thread blocks
-// per SM (the high-occupancy build: 7 for the pooled kernel, up to 72
-// registers; 8 for the lane-refill kernel, 64 registers).
+// per SM (launch_refill).
 // kPool selects how claimed rays reach idle lanes:
 //  * true: the whole warp tests each claimed chunk against the root box, two
 //    rays per lane, answers the misses at full width, and keeps the rays that
@@ -253,15 +252,22 @@ cudaError_t launch_persistent(const TraceArgs& t, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <int W, int kStack, int kMinBlocks, bool kAnalytic>
-cudaError_t launch_pooled(const TraceArgs& t, const LaunchParams& lp, cudaStream_t s) {
-    // High occupancy: the pooled kernel at 7 resident blocks per SM (up to 72
-    // registers: its split tail's state fits without spills; 8,063-8,070
-    // against 7,699-7,704 Mrays/s closest hit at 8 blocks), the lane-refill
-    // kernel at 8 (64 registers, no spills).
-    constexpr int kPooledBlocks = kMinBlocks >= 8 ? 7 : kMinBlocks;
-    return lp.root_pool ? launch_persistent<W, kStack, kPooledBlocks, kAnalytic, true>(t, s)
-                        : launch_persistent<W, kStack, kMinBlocks, kAnalytic, false>(t, s);
+// Persistent launch of either refill.  Accels of triangles alone always run
+// the kernel built for kOccupancyBlocks resident blocks per SM: its state fits
+// 72 registers without spills, and left to itself the compiler takes 117 to
+// 127 (4 blocks): 2,000,003 shadow rays on 1.3M triangles 183 against 220 us.
+// With analytic shapes in the leaf loop that build spills 200 to 250 bytes,
+// and the caller's flag decides.
+constexpr int kOccupancyBlocks = 7;
+template <int W, int kStack, bool kAnalytic>
+cudaError_t launch_refill(const TraceArgs& t, const LaunchParams& lp, cudaStream_t s) {
+    if constexpr (kAnalytic) {
+        if (!lp.high_occupancy)
+            return lp.root_pool ? launch_persistent<W, kStack, 1, kAnalytic, true>(t, s)
+                                : launch_persistent<W, kStack, 1, kAnalytic, false>(t, s);
+    }
+    return lp.root_pool ? launch_persistent<W, kStack, kOccupancyBlocks, kAnalytic, true>(t, s)
+                        : launch_persistent<W, kStack, kOccupancyBlocks, kAnalytic, false>(t, s);
 }
 
 template <int W, int kStack, bool kAnalytic>
@@ -285,12 +291,10 @@ cudaError_t launch_variant(const TraceArgs& t, const LaunchParams& lp, cudaStrea
                 else kc<<<(unsigned)blocks, block, 0, s>>>(q);
                 cudaError_t e = cudaGetLastError();
                 if (e != cudaSuccess) return e;
-                return lp.min_blocks >= 8 ? launch_pooled<W, kStack, 8, kAnalytic>(q, lp, s)
-                                          : launch_pooled<W, kStack, 1, kAnalytic>(q, lp, s);
+                return launch_refill<W, kStack, kAnalytic>(q, lp, s);
             }
         }
-        return lp.min_blocks >= 8 ? launch_pooled<W, kStack, 8, kAnalytic>(t, lp, s)
-                                  : launch_pooled<W, kStack, 1, kAnalytic>(t, lp, s);
+        return launch_refill<W, kStack, kAnalytic>(t, lp, s);
     }
     unsigned grid = (unsigned)((t.n + block - 1) / block);
     if (t.split_tail) {
