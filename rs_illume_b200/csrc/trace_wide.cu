@@ -37,6 +37,21 @@ __global__ void __launch_bounds__(128) k_trace_wide(TraceArgs a) {
     T.write(i, a);
 }
 
+// Rays a warp of k_trace_wide_split starts with, for n rays on a launch of
+// `threads` resident threads: the smallest power of two (at most 32) whose
+// warps are all resident at once.  The other lanes start idle and take
+// subtrees of the warp's rays, so fewer rays a warp shorten the longest ray's
+// chain of steps as long as the warps fit; beyond one wave they queue.
+// Measured us at 32 / 16 / chosen, camera rays on a 32,768-triangle soup:
+// 1,000 rays 79 / 55 / 29 (1 a warp), 10,000 94 / 64 / 41 (4), 33,000
+// 99 / 75 / 70 (8), and at half the chosen number 57 (10,000) and 91 (33,000);
+// incoherent rays gain 0 to 20 %.
+__host__ __device__ __forceinline__ uint32_t rays_per_warp(uint64_t n, uint64_t threads) {
+    uint32_t r = 1;
+    while (r < 32u && n * 32u > threads * r) r *= 2u;
+    return r;
+}
+
 // One thread per ray with the split tail from the start: a lane whose ray
 // missed the scene's root box or has finished takes subtrees of its warp's
 // unfinished rays (share_subtrees).  A one-wave query is all tail: its
@@ -56,7 +71,7 @@ __global__ void __launch_bounds__(128) k_trace_wide_split(TraceArgs a) {
     const uint64_t n = ray_count(a);
     if (a.small_max && n > a.small_max) return;   // the persistent launch beside this one has it
     const uint32_t warp_rays = a.warp_rays ? a.warp_rays
-                                           : (2 * n <= (uint64_t)gridDim.x * blockDim.x ? 16u : 32u);
+                                           : rays_per_warp(n, (uint64_t)gridDim.x * blockDim.x);
     const uint64_t warp_id = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t i = warp_id * warp_rays + lane;
     if (lane < warp_rays && i < n) {
@@ -278,15 +293,16 @@ cudaError_t launch_variant(const TraceArgs& t, const LaunchParams& lp, cudaStrea
             // A queue whose count is known on the device only: a count of at
             // most one wave of the split kernel runs there (all of its rays
             // resident at once, idle lanes helping from the start), a larger
-            // one on the persistent kernel.
+            // one on the persistent kernel.  The launch has a warp for every
+            // ray that the queue can hold, up to one wave.
             auto kc = k_trace_wide_split<W, kStack, false, kAnalytic>;
             auto ka = k_trace_wide_split<W, kStack, true, kAnalytic>;
             const uint64_t wave_blocks = resident_blocks(t.occ ? (const void*)ka : (const void*)kc, (int)block);
-            const uint64_t blocks = std::min<uint64_t>(wave_blocks, (t.n + block - 1) / block);
+            const uint64_t blocks = std::min<uint64_t>(wave_blocks, (t.n + block / 32 - 1) / (block / 32));
             if (blocks > 0) {
                 TraceArgs q = t;
                 q.small_max = blocks * block;
-                q.warp_rays = 0;                    // 16 rays a warp when the count allows
+                q.warp_rays = 0;                    // from the device-side count (rays_per_warp)
                 if (t.occ) ka<<<(unsigned)blocks, block, 0, s>>>(q);
                 else kc<<<(unsigned)blocks, block, 0, s>>>(q);
                 cudaError_t e = cudaGetLastError();
@@ -298,13 +314,11 @@ cudaError_t launch_variant(const TraceArgs& t, const LaunchParams& lp, cudaStrea
     }
     unsigned grid = (unsigned)((t.n + block - 1) / block);
     if (t.split_tail) {
-        // A query that fits half a wave starts each warp with 16 rays, so
-        // that half its lanes help from the first pass.
         auto kc = k_trace_wide_split<W, kStack, false, kAnalytic>;
         auto ka = k_trace_wide_split<W, kStack, true, kAnalytic>;
         const uint64_t wave = resident_blocks(t.occ ? (const void*)ka : (const void*)kc, (int)block) * block;
         TraceArgs q = t;
-        q.warp_rays = 2 * t.n <= wave ? 16u : 32u;
+        q.warp_rays = rays_per_warp(t.n, wave);
         const uint64_t rays_per_block = (uint64_t)q.warp_rays * (block / 32);
         const unsigned g = (unsigned)((t.n + rays_per_block - 1) / rays_per_block);
         if (t.occ) ka<<<g, block, 0, s>>>(q);
