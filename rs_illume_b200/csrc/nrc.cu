@@ -131,6 +131,14 @@ struct RowIn {
     float ps[3], pc[3];   // encoding state: the last octave's (sin, cos) per axis
 };
 
+// theta / pi of a unit vector's z, phi / 2 pi of its x and y.
+__device__ __forceinline__ float row_theta(float z) {
+    return acosf(fminf(fmaxf(z, -1.0f), 1.0f)) * (1.0f / 3.14159265358979f);
+}
+__device__ __forceinline__ float row_phi(float x, float y) {
+    return atan2f(y, x) * (0.5f / 3.14159265358979f) + 0.5f;
+}
+
 __device__ __forceinline__ RowIn load_row(const float* __restrict__ raw, uint32_t r, const Enc& e) {
     const float* p = raw + 12 * (size_t)r;
     RowIn v;
@@ -139,9 +147,8 @@ __device__ __forceinline__ RowIn load_row(const float* __restrict__ raw, uint32_
     v.q[2] = (p[2] - e.z0) * e.sz;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        float x = p[3 + 3 * k], y = p[4 + 3 * k], z = p[5 + 3 * k];
-        v.u[2 * k] = acosf(fminf(fmaxf(z, -1.0f), 1.0f)) * (1.0f / 3.14159265358979f);
-        v.u[2 * k + 1] = atan2f(y, x) * (0.5f / 3.14159265358979f) + 0.5f;
+        v.u[2 * k] = row_theta(p[5 + 3 * k]);
+        v.u[2 * k + 1] = row_phi(p[3 + 3 * k], p[4 + 3 * k]);
     }
     v.alb[0] = p[9];
     v.alb[1] = p[10];
@@ -480,103 +487,272 @@ __global__ void __launch_bounds__(128 * kTcGroups, 1) k_mlp_fwd_tc(const float* 
     tc_teardown(fail, tmem_base, err, mb, phase);
 }
 
-// ---------------------------------------------------------------- inference on tcgen05, two tiles per warpgroup
-// k_mlp_infer_tc: the inference forward with two 128-row tiles in flight per
-// warpgroup.  Each tile (slot) has its own A buffer (128 rows x 64 features,
-// 16 KB), its own 64 TMEM columns and its own mbarrier; the warpgroup
-// alternates between its slots, so while one slot's MMAs run the threads
-// produce the other slot's next A operand (encoding or accumulator -> ReLU ->
-// bf16).  Layer 0 is issued in four parts of K = 64, 64, 64 and 16 features
-// (features 0-63, 64-127, 128-191, 192-207), so an A buffer holds 64
-// features; a tile takes nine MMA batches (four layer-0 parts, five layers).
-// With 4 warpgroups per CTA, 8 tiles are in flight per SM (192,512 bytes of
-// shared memory, all 512 TMEM columns).  Waits are bounded; a warpgroup
-// whose wait gives up drains both slots' last commits before the TMEM is
-// freed.
-constexpr int kInfABytes = 128 / 8 * 8 * 128;                        // 16,384
-constexpr int kInfSmem = kTcWBytes + kTcGroups * 2 * kInfABytes;      // 192,512
+// ---------------------------------------------------------------- inference on tcgen05
+// k_mlp_infer_tc: the inference forward.  What it spends its time on is the
+// threads' work on the MMAs' A operands (encoding, accumulator -> bf16 ->
+// ReLU), so everything else is kept off that path:
+//  * A lives in TMEM (tcgen05.st; 32 columns hold a row's 64 bf16 features).
+//    From shared memory an MMA of N = 64 took about 100 cycles to issue, its
+//    A tile being four fifths of what it fetches; eight tiles in flight waited
+//    700 cycles and more for each batch of four.
+//  * Up to five 128-row tiles are in flight per SM, one per warpgroup, each
+//    with 64 accumulator and 32 operand columns (480 of the 512); thread t of
+//    a warpgroup owns row t.
+//  * No barriers: the last of a tile's four warps to finish its share of an
+//    operand (an acquire-release counter in shared memory) issues the batch
+//    and commits it to the tile's mbarrier, and each warp waits there by itself.
+// Layer 0 is issued in four parts of K = 64, 64, 64 and 16 features, so a tile
+// takes nine MMA batches.  727,329 rows: 136.5 us with two tiles per
+// warpgroup from shared memory and two barriers a batch, 77.8 us now (553 TFLOP/s,
+// 0.34 of the measured bf16 peak).
+// Waits are bounded; a warp whose wait gave up sets `fail`, which ends the
+// others' waits, and every tile's last commit is drained before the TMEM is
+// freed (see tc_teardown).
+constexpr int kInfGroups = 5;                   // warpgroups per CTA, at most
+constexpr uint32_t kInfCols = 96;               // TMEM columns per warpgroup: 64 accumulator, 32 operand
 
-// The features of layer-0 part p (groups 8p .. 8p + 7, at most 25) into
-// columns 0.. of an A buffer (8 core-matrix columns, SBO 1024).
-template <int KC, int KEND>
-__device__ __forceinline__ void encode_part(uint8_t* a, int c0, int row, RowIn& v) {
-    const uint4 q = feature_group<KC>(v);
-    *reinterpret_cast<uint4*>(a + ((row >> 3) * 8 + (KC - c0)) * 128 + (row & 7) * 16) = q;
-    if constexpr (KC + 1 < KEND) encode_part<KC + 1, KEND>(a, c0, row, v);
+// Row r's 12 inputs; by 16-byte loads where the array allows.
+__device__ __forceinline__ void load_raw(const float* __restrict__ raw, uint32_t r, bool vec, float (&p)[12]) {
+    const float* src = raw + 12 * (size_t)r;
+    if (vec) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(src) + k);
+            p[4 * k] = v.x; p[4 * k + 1] = v.y; p[4 * k + 2] = v.z; p[4 * k + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 12; ++k) p[k] = __ldg(src + k);
+    }
 }
 
-// Issues one batch (no wait): fences, group barrier, one thread issues and
-// commits to the slot's mbarrier.
-__device__ __forceinline__ void inf_issue(int g, int t, uint32_t tmem_d, uint32_t a_base, uint32_t a_sbo,
-                                          uint32_t w_base, uint32_t w_sbo, int k0, int ksteps, int n_out,
-                                          bool accumulate, uint32_t mbar) {
-    fence_proxy_async();
-    tc_fence_before();
-    group_sync(g);
-    if (t == 0) {
-        tc_fence_after();
-        const uint32_t idesc = idesc_bf16(128, n_out);
-        for (int k = 0; k < ksteps; ++k) {
-            const uint64_t da = umma_desc(a_base + (uint32_t)k * 256u, 128u, a_sbo);
-            const uint64_t db = umma_desc(w_base + (uint32_t)(k0 + k) * 256u, 128u, w_sbo);
-            umma(tmem_d, da, db, idesc, (accumulate || k > 0) ? 1u : 0u);
+// Octaves O0 .. O0 + 3 of an axis as four bf16 pairs, from octave O0 - 1 in
+// (s, c) (octave 0: from q); (s, c) becomes the last one.  The doubling is
+// feature_group's, each operation rounded by itself, except that c - s and
+// c + s of octave kFuse round once with the product that s is (kFuse < 0:
+// none).  Which octaves those are is what the compiler made of this kernel's
+// two-tile form; it is kept so that its answers stay the same to the last bit.
+template <int O0, int kFuse>
+__device__ __forceinline__ void octaves(float q, float& s, float& c, uint32_t (&w)[4]) {
+    float s1 = s, c1 = c;   // the octave before (s, c)
+    if constexpr (O0 == 0) {
+        sincospif(q, &s, &c);
+    } else {
+        const float s2 = __fmul_rn(__fmul_rn(2.0f, s), c), c2 = __fmul_rn(__fsub_rn(c, s), __fadd_rn(c, s));
+        s = s2;
+        c = c2;
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        w[t] = pack(s, c);
+        if (t == 3) break;
+        const float s2 = __fmul_rn(__fmul_rn(2.0f, s), c);
+        float lo, hi;
+        if (O0 + t == kFuse) {
+            lo = __fmaf_rn(__fmul_rn(-2.0f, s1), c1, c);
+            hi = __fmaf_rn(__fmul_rn(2.0f, s1), c1, c);
+        } else {
+            lo = __fsub_rn(c, s);
+            hi = __fadd_rn(c, s);
+        }
+        s1 = s;
+        c1 = c;
+        s = s2;
+        c = __fmul_rn(lo, hi);
+    }
+}
+
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c),
+                 "r"(d)
+                 : "memory");
+}
+
+// Feature group KC >= 9 of a row into its operand columns.
+template <int KC>
+__device__ __forceinline__ void put_group(uint32_t tmem_a, RowIn& v) {
+    const uint4 q = feature_group<KC>(v);
+    tmem_st4(tmem_a + 4 * (KC & 7), q.x, q.y, q.z, q.w);
+}
+template <int KC, int KEND>
+__device__ __forceinline__ void put_groups(uint32_t tmem_a, RowIn& v) {
+    put_group<KC>(tmem_a, v);
+    if constexpr (KC + 1 < KEND) put_groups<KC + 1, KEND>(tmem_a, v);
+}
+
+// Part 0 of layer 0 (groups 0-7): axes 0 and 1 and the first 8 octaves of axis
+// 2, whose last one stays in the row state.
+template <bool kOdd>
+__device__ __forceinline__ void put_positions(uint32_t tmem_a, RowIn& v) {
+    uint32_t w[4];
+    float s = 0.0f, c = 0.0f;
+    octaves<0, -1>(v.q[0], s, c, w);
+    tmem_st4(tmem_a, w[0], w[1], w[2], w[3]);
+    octaves<4, -1>(0.0f, s, c, w);
+    tmem_st4(tmem_a + 4, w[0], w[1], w[2], w[3]);
+    octaves<8, kOdd ? 9 : -1>(0.0f, s, c, w);
+    tmem_st4(tmem_a + 8, w[0], w[1], w[2], w[3]);
+    octaves<0, -1>(v.q[1], s, c, w);
+    tmem_st4(tmem_a + 12, w[0], w[1], w[2], w[3]);
+    octaves<4, -1>(0.0f, s, c, w);
+    tmem_st4(tmem_a + 16, w[0], w[1], w[2], w[3]);
+    octaves<8, kOdd ? 9 : 8>(0.0f, s, c, w);
+    tmem_st4(tmem_a + 20, w[0], w[1], w[2], w[3]);
+    octaves<0, -1>(v.q[2], s, c, w);
+    tmem_st4(tmem_a + 24, w[0], w[1], w[2], w[3]);
+    octaves<4, -1>(0.0f, s, c, w);
+    tmem_st4(tmem_a + 28, w[0], w[1], w[2], w[3]);
+    v.ps[2] = s;
+    v.pc[2] = c;
+}
+
+// A row's share of layer-0 part `part` (groups 8 part .. 8 part + 7, at most 25).
+__device__ __forceinline__ void encode_part(int part, bool odd, uint32_t tmem_a, const float* __restrict__ raw,
+                                            uint32_t r, bool in_range, bool vec, const Enc& e, RowIn& v) {
+    if (part == 0) {
+        v = RowIn{};
+        if (in_range) {
+            float p[12];
+            load_raw(raw, r, vec, p);
+            v.q[0] = (p[0] - e.x0) * e.sx;
+            v.q[1] = (p[1] - e.y0) * e.sy;
+            v.q[2] = (p[2] - e.z0) * e.sz;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                v.u[2 * k] = row_theta(p[5 + 3 * k]);
+                v.u[2 * k + 1] = row_phi(p[3 + 3 * k], p[4 + 3 * k]);
+            }
+            v.alb[0] = p[9];
+            v.alb[1] = p[10];
+            v.alb[2] = p[11];
+        }
+        if (odd) put_positions<true>(tmem_a, v);
+        else put_positions<false>(tmem_a, v);
+    } else if (part == 1) {
+        uint32_t w[4];
+        octaves<8, -1>(0.0f, v.ps[2], v.pc[2], w);
+        tmem_st4(tmem_a, w[0], w[1], w[2], w[3]);
+        put_groups<9, 16>(tmem_a, v);
+    } else if (part == 2) {
+        put_groups<16, 24>(tmem_a, v);
+    } else {
+        put_groups<24, 26>(tmem_a, v);
+    }
+}
+
+// Accumulator row (64 columns) -> bf16 -> ReLU -> its operand columns.
+// Rounding is monotone, so the packed maximum with zero gives what the ReLU
+// before it gives, in half the instructions.
+__device__ __forceinline__ void acc_to_operand(uint32_t tmem_d, uint32_t tmem_a) {
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t r[32];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,"
+            "%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+              "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+            : "r"(tmem_d + 32u * h));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        uint32_t w[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const __nv_bfloat162 b =
+                __hmax2(__floats2bfloat162_rn(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1])), zero);
+            w[k] = *reinterpret_cast<const uint32_t*>(&b);
+        }
+        asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
+                tmem_a + 16u * h),
+            "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]),
+            "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
+            : "memory");
+    }
+}
+
+// One MMA with A in TMEM; B's descriptor by its low word (start address, LBO)
+// and high word (SBO, version).
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                        uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tmov.b64 db, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}\n"
+        :
+        : "r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+// Issues batch k (0-3: the parts of layer 0, 4-8: layers 1-5) of a tile and
+// commits it to the tile's mbarrier; called by a whole warp, whose lane 0
+// issues.  A K-step is 8 operand columns and 256 bytes of weights.
+__device__ __forceinline__ void inf_issue(int k, uint32_t tmem_d, uint32_t tmem_a, uint32_t w_base, uint32_t mbar,
+                                          uint32_t lane) {
+    constexpr uint32_t kLbo = (128u >> 4) << 16;
+    constexpr uint32_t kHi8 = (8u * 128u >> 4) | (1u << 14), kHi26 = (26u * 128u >> 4) | (1u << 14);
+    const int l = k < 4 ? 0 : k - 3;
+    const uint32_t w_at = w_base + 2u * (l == 0 ? 0u : (uint32_t)(kHid * kIn + (l - 1) * kHid * kHid)) +
+                          (k < 4 ? (uint32_t)k * 1024u : 0u);
+    const uint32_t b_lo = (w_at >> 4) | kLbo, b_hi = l == 0 ? kHi26 : kHi8;
+    const uint32_t idesc = k == 8 ? idesc_bf16(128, 16) : idesc_bf16(128, 64);
+    tc_fence_after();
+    if (lane == 0) {
+        umma_ts(tmem_d, tmem_a, b_lo, b_hi, idesc, k > 0 && k < 4 ? 1u : 0u);
+        if (k != 3) {
+            umma_ts(tmem_d, tmem_a + 8u, b_lo + 16u, b_hi, idesc, 1u);
+            umma_ts(tmem_d, tmem_a + 16u, b_lo + 32u, b_hi, idesc, 1u);
+            umma_ts(tmem_d, tmem_a + 24u, b_lo + 48u, b_hi, idesc, 1u);
         }
         umma_commit(mbar);
     }
 }
 
-// Waits for the slot's last batch (issuing thread, bounded); false on a timeout.
-__device__ __forceinline__ bool inf_wait(int g, int t, uint32_t mbar, uint32_t& phase, volatile int* fail) {
-    if (t == 0) {
-        uint32_t it = 0;
-        while (!mbar_try_wait(mbar, phase) && ++it < kTcWaitCap) {}
-        if (it >= kTcWaitCap) *fail = 1;
-    }
-    phase ^= 1u;
-    group_sync(g);
-    tc_fence_after();
-    return *fail == 0;
-}
-
-// Batch k (0-8) of the slot's tile: its A operand, then the issue.
-__device__ __forceinline__ void inf_step(int k, int g, int t, uint8_t* a, uint32_t a_base, uint32_t w_base,
-                                         uint32_t tmem_d, uint32_t tmem_row, RowIn& v, uint32_t mbar) {
-    if (k < 4) {
-        switch (k) {
-            case 0: encode_part<0, 8>(a, 0, t, v); break;
-            case 1: encode_part<8, 16>(a, 8, t, v); break;
-            case 2: encode_part<16, 24>(a, 16, t, v); break;
-            default: encode_part<24, 26>(a, 24, t, v); break;
+// A warp's bounded wait for a phase; false (for the whole warp) when it or
+// another warp gave up.
+__device__ __forceinline__ bool warp_wait(uint32_t mbar, uint32_t parity, volatile int* fail) {
+    bool ok = true;
+    uint32_t it = 0;
+    while (!mbar_try_wait(mbar, parity)) {
+        if (++it >= kTcWaitCap || *fail) {
+            *fail = 1;
+            ok = false;
+            break;
         }
-        inf_issue(g, t, tmem_d, a_base, 8 * 128, w_base + 2 * param_off(0), 26 * 128, 4 * k, k < 3 ? 4 : 1, 64,
-                  k > 0, mbar);
-    } else {
-        const int l = k - 3;
-        acc_to_a(tmem_row, a, t, nullptr);
-        inf_issue(g, t, tmem_d, a_base, 8 * 128, w_base + 2 * param_off(l), 8 * 128, 0, 4, l == 5 ? 16 : 64, false,
-                  mbar);
     }
+    ok = __all_sync(0xFFFFFFFFu, ok);
+    tc_fence_after();
+    return ok;
 }
 
-__global__ void __launch_bounds__(128 * kTcGroups, 1) k_mlp_infer_tc(const float* __restrict__ raw, NrcCount cnt,
-                                                                     Enc ec, const __nv_bfloat16* __restrict__ wtc,
-                                                                     float* __restrict__ out, uint32_t* err) {
+__global__ void __launch_bounds__(128 * kInfGroups, 1) k_mlp_infer_tc(const float* __restrict__ raw, NrcCount cnt, Enc ec,
+                                                                      const __nv_bfloat16* __restrict__ wtc,
+                                                                      float* __restrict__ out, uint32_t* err,
+                                                                      uint32_t tmem_cols) {
     extern __shared__ __align__(1024) uint8_t tc_smem[];
-    __shared__ __align__(8) uint64_t mbar[2 * kTcGroups];
-    __shared__ int fail[kTcGroups];
+    __shared__ __align__(8) uint64_t mbar[kInfGroups];   // a warpgroup's last batch is done
+    __shared__ __align__(8) uint64_t wbar;               // the weights are here
+    __shared__ uint32_t arrived[kInfGroups];             // warps that finished their share, ever
+    __shared__ uint32_t issued[kInfGroups];              // batches issued, ever
+    __shared__ int fail;
     __shared__ uint32_t tmem_base;
-    const int warp = threadIdx.x >> 5, g = warp >> 2, t = threadIdx.x & 127;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);   // uniform, and known to be
+    const int g = warp >> 2;
+    const uint32_t lane = threadIdx.x & 31u, t = threadIdx.x & 127u;
     const uint32_t groups = blockDim.x >> 7;
-    {
-        const uint4* src = reinterpret_cast<const uint4*>(wtc);
-        uint4* dst = reinterpret_cast<uint4*>(tc_smem);
-        for (int k = threadIdx.x; k < kTcWBytes / 16; k += blockDim.x) dst[k] = src[k];
+    if (threadIdx.x < groups) {
+        mbar_init(smem_u32(&mbar[threadIdx.x]));
+        arrived[threadIdx.x] = 0;
+        issued[threadIdx.x] = 0;
     }
-    if (threadIdx.x < 2 * groups) mbar_init(smem_u32(&mbar[threadIdx.x]));
-    if (threadIdx.x < groups) fail[threadIdx.x] = 0;
+    if (threadIdx.x == 0) {
+        mbar_init(smem_u32(&wbar));
+        fail = 0;
+    }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                     "r"(128u * groups));
+                     "r"(tmem_cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -584,73 +760,89 @@ __global__ void __launch_bounds__(128 * kTcGroups, 1) k_mlp_infer_tc(const float
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (threadIdx.x == 0) {   // the weights, while the first tiles are encoded
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&wbar)), "r"(kTcWBytes)
+                     : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         smem_u32(tc_smem)),
+                     "l"(wtc), "r"(kTcWBytes), "r"(smem_u32(&wbar))
+                     : "memory");
+    }
     const uint32_t n = rows_of(cnt);
-    const uint32_t w_base = smem_u32(tc_smem);
-    // per slot: A buffer, TMEM columns (and this warp's lanes), mbarrier
-    auto a_of = [&](int sl) { return tc_smem + kTcWBytes + (2 * g + sl) * kInfABytes; };
-    auto tmem_of = [&](int sl) { return tmem_base + 64u * (2u * g + sl); };
-    auto lanes_of = [&](int sl) { return tmem_of(sl) + ((uint32_t)(32 * (warp & 3)) << 16); };
-    auto mb_of = [&](int sl) { return smem_u32(&mbar[2 * g + sl]); };
-    uint32_t phase[2] = {0u, 0u};
-    // a committed batch not yet waited for, and its phase parity
-    bool pending[2] = {false, false};
-    uint32_t pend_par[2] = {0u, 0u};
-    const uint32_t tiles = (n + 127) / 128, pairs = (tiles + 1) / 2;
-    bool ok = true;
-    for (uint32_t pr = blockIdx.x * groups + g; pr < pairs && ok; pr += gridDim.x * groups) {
-        RowIn v[2];
-#pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
-            const uint32_t row = (2 * pr + sl) * 128 + t;
-            v[sl] = RowIn{};
-            if (row < n) v[sl] = load_row(raw, row, ec);
-        }
-        for (int k = 0; k < 9 && ok; ++k) {
-#pragma unroll
-            for (int sl = 0; sl < 2; ++sl) {
-                if (k > 0) {
-                    ok = inf_wait(g, t, mb_of(sl), phase[sl], &fail[g]);
-                    if (!ok) break;
-                    pending[sl] = false;
-                }
-                pend_par[sl] = phase[sl];
-                uint8_t* buf = a_of(sl);
-                inf_step(k, g, t, buf, smem_u32(buf), w_base, tmem_of(sl), lanes_of(sl), v[sl], mb_of(sl));
-                pending[sl] = true;
+    const bool vec = ((uintptr_t)raw & 15u) == 0;
+    const uint32_t tmem_d = tmem_base + kInfCols * g, tmem_a = tmem_d + 64u;   // the MMAs' addresses
+    const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;                  // this warp's rows of them
+    const uint32_t mb = smem_u32(&mbar[g]);
+    const uint32_t tiles = (n + 127) / 128;
+    uint32_t parity = 0;
+    bool ok = true, weights_here = false;
+    for (uint32_t tile = blockIdx.x * groups + g; tile < tiles && ok; tile += gridDim.x * groups) {
+        const uint32_t r = tile * 128u + t;
+        RowIn v;
+        for (int k = 0; k < 9; ++k) {
+            if (k > 0) {
+                ok = warp_wait(mb, parity, &fail);
+                parity ^= 1u;
+                if (!ok) break;
             }
+            if (k < 4) encode_part(k, (tile & 1u) != 0, tmem_a + lanes, raw, r, r < n, vec, ec, v);
+            else acc_to_operand(tmem_d + lanes, tmem_a + lanes);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();     // accumulator reads and operand writes, ordered before the MMAs
+            __syncwarp();
+            uint32_t before = 0;
+            if (lane == 0)
+                asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
+                             : "=r"(before)
+                             : "r"(smem_u32(&arrived[g]))
+                             : "memory");
+            before = __shfl_sync(0xFFFFFFFFu, before, 0);
+            if ((before & 3u) == 3u) {   // the operand is complete
+                if (!weights_here) {
+                    uint32_t it = 0;
+                    while (!mbar_try_wait(smem_u32(&wbar), 0u) && ++it < kTcWaitCap) {}
+                    if (it >= kTcWaitCap) fail = 1;
+                    weights_here = true;
+                }
+                if (lane == 0) issued[g] += 1;
+                inf_issue(k, tmem_d, tmem_a, smem_u32(tc_smem), mb, lane);
+            }
+            __syncwarp();
         }
         if (!ok) break;
-#pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
-            ok = ok && inf_wait(g, t, mb_of(sl), phase[sl], &fail[g]);
-            if (!ok) break;
-            pending[sl] = false;
-            float o[16];
-            tmem_ld16(lanes_of(sl), o);
-            const uint32_t row = (2 * pr + sl) * 128 + t;
-            if (row < n) {
-                out[3 * (size_t)row] = o[0];
-                out[3 * (size_t)row + 1] = o[1];
-                out[3 * (size_t)row + 2] = o[2];
-            }
+        ok = warp_wait(mb, parity, &fail);
+        parity ^= 1u;
+        if (!ok) break;
+        float o[16];
+        tmem_ld16(tmem_d + lanes, o);
+        tc_fence_before();   // the next tile's batches overwrite the columns
+        if (r < n) {
+            out[3 * (size_t)r] = o[0];
+            out[3 * (size_t)r + 1] = o[1];
+            out[3 * (size_t)r + 2] = o[2];
         }
-    }
-    // a wait that gave up: drain both slots' outstanding commits, then
-    // report; see tc_teardown
-    if (t == 0 && fail[g]) {
-#pragma unroll
-        for (int sl = 0; sl < 2; ++sl) {
-            if (!pending[sl]) continue;
-            uint32_t it = 0;
-            while (!mbar_try_wait(mb_of(sl), pend_par[sl]) && ++it < kTcDrainCap) {}
-        }
-        atomicOr(err, kErrMlpTimeout);
     }
     tc_fence_before();
     __syncthreads();
+    if (threadIdx.x == 0) {
+        tc_fence_after();
+        // the weights' copy and every warpgroup's last batch, before shared
+        // memory and TMEM are given back
+        uint32_t it = 0;
+        while (!mbar_try_wait(smem_u32(&wbar), 0u) && ++it < kTcDrainCap) {}
+        if (fail) {
+            for (uint32_t q = 0; q < groups; ++q) {
+                if (issued[q] == 0) continue;
+                it = 0;
+                while (!mbar_try_wait(smem_u32(&mbar[q]), (issued[q] - 1u) & 1u) && ++it < kTcDrainCap) {}
+            }
+            atomicOr(err, kErrMlpTimeout);
+        }
+    }
+    __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(128u * groups));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols));
     }
 }
 
@@ -1076,11 +1268,14 @@ cudaError_t forward(ilm_nrc* h, const float* raw, NrcCount cnt, bool train, floa
             raw, cnt, enc_params(h), static_cast<const __nv_bfloat16*>(h->wtc.ptr), out, err, rows,
             static_cast<__nv_bfloat16*>(h->acts.ptr), static_cast<__nv_bfloat16*>(h->enc.ptr));
     else {
-        // inference: two tiles per warpgroup, 4 warpgroups per CTA, one CTA per SM
-        const uint32_t pairs = (rows + 255) / 256;   // two 128-row tiles per pair
-        const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(148, (pairs + kTcGroups - 1) / kTcGroups));
-        k_mlp_infer_tc<<<grid, 128 * kTcGroups, kInfSmem, s>>>(
-            raw, cnt, enc_params(h), static_cast<const __nv_bfloat16*>(h->winf.ptr), out, err);
+        // one CTA per SM, a warpgroup for every tile as long as there are SMs
+        // and warpgroups; TMEM columns are allocated in powers of two
+        const uint32_t tiles = std::max<uint32_t>(1, (rows + 127) / 128);
+        const uint32_t groups = std::min<uint32_t>(kInfGroups, (tiles + 147) / 148);
+        const uint32_t grid = std::min<uint32_t>(148, (tiles + groups - 1) / groups);
+        const uint32_t cols = groups == 1 ? 128u : (groups == 2 ? 256u : 512u);
+        k_mlp_infer_tc<<<grid, 128 * groups, kTcWBytes, s>>>(
+            raw, cnt, enc_params(h), static_cast<const __nv_bfloat16*>(h->winf.ptr), out, err, cols);
     }
     return cudaGetLastError();
 }
@@ -1192,10 +1387,9 @@ int32_t ilm_nrc_create(ilm_context* ctx, const ilm_nrc_config* cfg, ilm_nrc** ou
     cudaMemset(h->winf.ptr, 0, kParams * 2);
     cudaMemset(h->wtcb.ptr, 0, kTcbElems * 2);
     cudaFuncSetAttribute(k_mlp_fwd_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-    cudaFuncSetAttribute(k_mlp_fwd_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
     cudaFuncSetAttribute(k_mlp_bwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcbSmem);
     cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
-    cudaFuncSetAttribute(k_mlp_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfSmem);
+    cudaFuncSetAttribute(k_mlp_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcWBytes);
     if ((e = pack(h.get(), h->stream)) != cudaSuccess) return cuda_fail(ctx, e, "nrc pack");
     if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return cuda_fail(ctx, e, "nrc");
     *out = h.release();
