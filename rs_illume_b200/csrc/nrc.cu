@@ -11,18 +11,16 @@
 //   loss = mean over samples and channels of (p - y)^2 / (sg(p)^2 + 0.01).
 //
 // Kernels
-//   k_mlp_fwd_tc<train>  forward pass: per 128-row tile a warpgroup encodes its
-//                  rows straight into layer 0's A operand in shared memory,
-//                  one thread issues the MMAs, each layer's accumulator comes
-//                  back through tcgen05.ld as the next layer's A; training
-//                  also stores the encoding and the bf16 activations
-//   k_mlp_bwd_tc   loss gradient, then back through the layers the same way
-//                  (transposed weights), storing dOut
+//   k_mlp_infer_tc inference: per 128-row tile a warpgroup encodes its rows
+//                  into TMEM as layer 0's A operand, one thread issues the
+//                  MMAs, each layer's accumulator becomes the next A
+//   k_mlp_train_tc training: the same forward, then the loss gradient and the
+//                  way back through the layers (transposed weights); stores
+//                  the encoding, the bf16 activations and dOut
 //   k_wgrad_tc     dW_l = dOut_l^T * in_l for all six layers on tcgen05
 //                  (M = outputs, N = inputs, K = batch rows, both operands
-//                  MN-major as the rows are stored, staged by 16-byte
-//                  cp.async into two buffers); split-K over the rows, one FP32
-//                  partial per CTA, no atomics
+//                  MN-major as the rows are stored, staged by bulk copies);
+//                  split-K over the rows, one FP32 partial per chunk, no atomics
 //   k_reduce_adam  sums the CTA partials, Adam on the FP32 master weights,
 //                  bf16 weight packs and the inference moving average
 //   k_nrc_encode   the encoding alone (for inspection)
@@ -69,7 +67,6 @@ __host__ __device__ constexpr int tcb_index(int l, int o, int i) {
 }
 constexpr int kTcbElems = 4 * kHid * kHid + kHid * kOut;   // 17408
 constexpr float kLossEps = 0.01f;
-constexpr int kMaxPartials = 148;   // CTAs of k_wgrad_tc (one FP32 partial gradient each)
 
 struct Enc {   // position normalisation: q = (p - origin) * scale
     float x0, y0, z0, sx, sy, sz;
@@ -98,30 +95,10 @@ __device__ __forceinline__ uint32_t rows_of(const NrcCount& c) {
     return n;
 }
 
-// 16-byte global -> shared copy; zero-filled when !ok.
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok) {
-    uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    int sz = ok ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(sz));
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
-
 __device__ __forceinline__ uint32_t pack(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
-__device__ __forceinline__ float lo_of(uint32_t p) { return __uint_as_float(p << 16); }
-__device__ __forceinline__ float hi_of(uint32_t p) { return __uint_as_float(p & 0xFFFF0000u); }
-
-// Copies n bf16 (a multiple of 8) from global to shared memory with 16-byte loads.
-__device__ __forceinline__ void stage(__nv_bfloat16* dst, const __nv_bfloat16* src, int n) {
-    const uint4* s = reinterpret_cast<const uint4*>(src);
-    uint4* d = reinterpret_cast<uint4*>(dst);
-    for (int i = threadIdx.x; i < n / 8; i += blockDim.x) d[i] = s[i];
-}
-
 // ---------------------------------------------------------------- encoding
 // What the encoder needs of one input row.
 struct RowIn {
@@ -235,30 +212,20 @@ __global__ void k_nrc_encode(const float* __restrict__ raw, uint32_t n, Enc ec, 
     encode_row<0>(v, reinterpret_cast<uint32_t*>(enc + (size_t)i * kIn));
 }
 
-// ---------------------------------------------------------------- forward on tcgen05
-// k_mlp_fwd_tc: the forward pass on the 5th-generation tensor cores.
-// A CTA of 1, 2 or 4 warpgroups (blockDim / 128; few per CTA for small
-// batches, so that the tiles spread over the SMs); each warpgroup owns 128-row tiles (thread t
-// = row t), its own A operand buffer in shared memory, 64 TMEM columns of
-// FP32 accumulator (rows = TMEM lanes) and an mbarrier.  Per tile:
-//   layer 0 in two K halves (features 0-111, 112-207): the threads evaluate
-//     their row's encoding into A, one thread issues tcgen05.mma
-//     (M 128, N 64, K 16, bf16 x bf16 -> f32) and commits to the mbarrier;
-//   layers 1-4: tcgen05.ld of the accumulator, ReLU, bf16 into A, MMA;
-//   layer 5: N = 16, the first 3 columns are the output.
-// Training also stores each row's encoding ([n][208] bf16) and its five
-// ReLU'd activations (layer l at acts + l * ld * 64, [n][64] bf16), the bf16
-// values that go into the next layer's A operand.
-// The weights (61,440 bytes, all layers) are staged once per CTA.  Operands
-// use the canonical K-major layout without swizzle: 8x8 core matrices of 128
-// contiguous bytes; LBO = 128 bytes (next core matrix along K), SBO = the
-// stride between 8-row groups.  Every mbarrier wait is bounded; a timeout
-// sets kErrMlpTimeout in *err and the warpgroup stops.
-constexpr int kTcGroups = 4;                                   // warpgroups per CTA, at most
-constexpr int kTcHalfCols = 14;                                // core-matrix columns of an A buffer (112 features)
-constexpr int kTcABytes = 128 / 8 * kTcHalfCols * 128;         // 28,672
-constexpr int kTcWBytes = kParams * 2;                         // 61,440
-constexpr int kTcSmem = kTcWBytes + kTcGroups * kTcABytes;     // 176,128 at 4 warpgroups
+// ---------------------------------------------------------------- tcgen05
+// The network's layers are D = A * W^T on the 5th-generation tensor cores: A
+// 128 rows of bf16 operands in TMEM, W in shared memory, FP32 D in TMEM.  The
+// weight packs use the canonical K-major layout without swizzle: 8x8 core
+// matrices of 128 contiguous bytes; LBO = 128 bytes (next core matrix along
+// K), SBO = the stride between 8-row groups.  Every mbarrier wait is bounded;
+// a timeout sets kErrMlpTimeout in *err.  Waits that gave up are followed by
+// a drain, up to kTcDrainCap more polls on the last commit's phase, so that
+// tcgen05.dealloc does not free columns an MMA may still write.  If the drain
+// runs out too, the columns are freed all the same -- a CTA that kept them
+// would leave the tcgen05.alloc of later CTAs on its SM waiting -- and the
+// error word marks the launch's results as invalid.
+constexpr int kTcWBytes = kParams * 2;                         // 61,440: all layers' forward weights
+constexpr int kTcbWBytes = kTcbElems * 2;                      // 34,816: the transposed ones, layers 1-5
 constexpr uint32_t kErrMlpTimeout = 4u;
 constexpr uint32_t kTcWaitCap = 1u << 22;   // try_wait polls before a wait gives up
 constexpr uint32_t kTcDrainCap = 1u << 26;  // further polls for a batch whose wait gave up
@@ -301,9 +268,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t mbar, uint32_t parity) {
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void group_sync(int g) {
-    asm volatile("bar.sync %0, 128;" ::"r"(g + 1) : "memory");
-}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
     asm volatile(
@@ -315,176 +279,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
     for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
-
-// Row t's 8 features F..F+7 (F = 8 * KC) into core-matrix column c of an A
-// buffer, and into the row's stored encoding when genc is set.
-template <int KC>
-__device__ __forceinline__ void put_features(uint8_t* a, int c, int row, RowIn& v, uint4* genc) {
-    const uint4 q = feature_group<KC>(v);
-    *reinterpret_cast<uint4*>(a + ((row >> 3) * kTcHalfCols + c) * 128 + (row & 7) * 16) = q;
-    if (genc) genc[KC] = q;
-}
-template <int KC, int KEND>
-__device__ __forceinline__ void encode_cols(uint8_t* a, int c0, int row, RowIn& v, uint4* genc) {
-    put_features<KC>(a, KC - c0, row, v, genc);
-    if constexpr (KC + 1 < KEND) encode_cols<KC + 1, KEND>(a, c0, row, v, genc);
-}
-
-// One warpgroup's MMA batch: layer with `ksteps` K-steps of 16, A from
-// `a_base` (SBO a_sbo), B = layer weights from `w_base` (SBO w_sbo) starting at
-// K-step k0; then commit and (thread 0) wait.  Returns false on a timeout.
-__device__ __forceinline__ bool mma_batch(int g, int t, uint32_t tmem_d, uint32_t a_base, uint32_t a_sbo,
-                                          uint32_t w_base, uint32_t w_sbo, int k0, int ksteps, int n_out,
-                                          bool accumulate, uint32_t mbar, uint32_t& phase, volatile int* fail) {
-    fence_proxy_async();   // the A tile written by this warpgroup, visible to the tensor core
-    tc_fence_before();     // the accumulator reads above, ordered before the MMAs below
-    group_sync(g);
-    if (t == 0) {
-        tc_fence_after();
-        const uint32_t idesc = idesc_bf16(128, n_out);
-        for (int k = 0; k < ksteps; ++k) {
-            uint64_t da = umma_desc(a_base + (uint32_t)k * 256u, 128u, a_sbo);
-            uint64_t db = umma_desc(w_base + (uint32_t)(k0 + k) * 256u, 128u, w_sbo);
-            umma(tmem_d, da, db, idesc, (accumulate || k > 0) ? 1u : 0u);
-        }
-        umma_commit(mbar);
-        uint32_t it = 0;
-        while (!mbar_try_wait(mbar, phase) && ++it < kTcWaitCap) {}
-        if (it >= kTcWaitCap) *fail = 1;
-    }
-    phase ^= 1u;
-    group_sync(g);
-    tc_fence_after();
-    return *fail == 0;
-}
-
-// Accumulator row t (64 columns) -> ReLU -> bf16 A operand (K = 64, SBO 1024),
-// and into the row's stored activation ([64] bf16) when gact is set.
-__device__ __forceinline__ void acc_to_a(uint32_t tmem_row, uint8_t* a, int row, uint4* gact) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        float v[16];
-        tmem_ld16(tmem_row + 16 * q, v);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            uint4 w;
-            w.x = pack(fmaxf(v[8 * h], 0.0f), fmaxf(v[8 * h + 1], 0.0f));
-            w.y = pack(fmaxf(v[8 * h + 2], 0.0f), fmaxf(v[8 * h + 3], 0.0f));
-            w.z = pack(fmaxf(v[8 * h + 4], 0.0f), fmaxf(v[8 * h + 5], 0.0f));
-            w.w = pack(fmaxf(v[8 * h + 6], 0.0f), fmaxf(v[8 * h + 7], 0.0f));
-            *reinterpret_cast<uint4*>(a + ((row >> 3) * 8 + 2 * q + h) * 128 + (row & 7) * 16) = w;
-            if (gact) gact[2 * q + h] = w;
-        }
-    }
-}
-
-// TMEM, barriers and failure flags of a tcgen05 MLP kernel: allocation of
-// 64 columns per warpgroup (64, 128 or 256: powers of two) by warp 0 and the
-// fences that publish them.
-__device__ __forceinline__ void tc_setup(uint64_t* mbar, int* fail, uint32_t* tmem_base) {
-    const uint32_t groups = blockDim.x >> 7;
-    if (threadIdx.x < groups) {
-        mbar_init(smem_u32(&mbar[threadIdx.x]));
-        fail[threadIdx.x] = 0;
-    }
-    if ((threadIdx.x >> 5) == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base)),
-                     "r"(64u * groups));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-}
-
-// Reports a timed-out wait and frees the TMEM.  Every warpgroup has stopped
-// issuing by then: its last batch was committed and waited for, or its wait
-// gave up.  A warpgroup whose wait gave up first drains that batch: its issuing
-// thread waits again, up to kTcDrainCap more polls, on the same mbarrier phase
-// (the parity before mma_batch's flip, phase ^ 1), so tcgen05.dealloc does not
-// free columns an MMA may still write.  If the drain runs out too, the columns
-// are freed all the same -- a CTA that kept them would leave the tcgen05.alloc
-// of later CTAs on its SM waiting -- and the error word marks the launch's
-// results as invalid.  The CTA barrier below follows every warpgroup's exit.
-__device__ __forceinline__ void tc_teardown(const int* fail, uint32_t tmem_base, uint32_t* err, uint32_t mbar,
-                                            uint32_t phase) {
-    const int g = threadIdx.x >> 7;
-    if ((threadIdx.x & 127) == 0 && fail[g]) {
-        uint32_t it = 0;
-        while (!mbar_try_wait(mbar, phase ^ 1u) && ++it < kTcDrainCap) {}
-        atomicOr(err, kErrMlpTimeout);
-    }
-    tc_fence_before();
-    __syncthreads();
-    if ((threadIdx.x >> 5) == 0) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                     "r"(64u * (blockDim.x >> 7)));
-    }
-}
-
-template <bool kTrain>
-__global__ void __launch_bounds__(128 * kTcGroups, 1) k_mlp_fwd_tc(const float* __restrict__ raw, NrcCount cnt,
-                                                                   Enc ec, const __nv_bfloat16* __restrict__ wtc,
-                                                                   float* __restrict__ out, uint32_t* err,
-                                                                   uint32_t ld, __nv_bfloat16* __restrict__ acts,
-                                                                   __nv_bfloat16* __restrict__ enc) {
-    extern __shared__ __align__(1024) uint8_t tc_smem[];
-    __shared__ __align__(8) uint64_t mbar[kTcGroups];
-    __shared__ int fail[kTcGroups];
-    __shared__ uint32_t tmem_base;
-    const int warp = threadIdx.x >> 5, g = warp >> 2, t = threadIdx.x & 127;
-    // stage the weights; barriers; TMEM (64 columns per warpgroup)
-    {
-        const uint4* src = reinterpret_cast<const uint4*>(wtc);
-        uint4* dst = reinterpret_cast<uint4*>(tc_smem);
-        for (int k = threadIdx.x; k < kTcWBytes / 16; k += blockDim.x) dst[k] = src[k];
-    }
-    tc_setup(mbar, fail, &tmem_base);
-    const uint32_t n = rows_of(cnt);
-    const uint32_t tmem_d = tmem_base + 64u * g;                          // this warpgroup's columns
-    const uint32_t tmem_row = tmem_d + ((uint32_t)(32 * (warp & 3)) << 16);   // this warp's lanes
-    uint8_t* a = tc_smem + kTcWBytes + g * kTcABytes;
-    const uint32_t a_base = smem_u32(a), w_base = smem_u32(tc_smem);
-    const uint32_t mb = smem_u32(&mbar[g]);
-    uint32_t phase = 0;
-    const uint32_t tiles = (n + 127) / 128;
-    const uint32_t groups = blockDim.x >> 7;
-    for (uint32_t tile = blockIdx.x * groups + g; tile < tiles; tile += gridDim.x * groups) {
-        const uint32_t row = tile * 128 + t;
-        const bool keep = kTrain && row < n;
-        RowIn v = {};
-        if (row < n) v = load_row(raw, row, ec);
-        uint4* genc = keep ? reinterpret_cast<uint4*>(enc + (size_t)row * kIn) : nullptr;
-        // layer 0, features 0-111 (K-steps 0-6)
-        encode_cols<0, kTcHalfCols>(a, 0, t, v, genc);
-        if (!mma_batch(g, t, tmem_d, a_base, kTcHalfCols * 128, w_base + 2 * param_off(0), 26 * 128, 0, 7, 64,
-                       false, mb, phase, &fail[g]))
-            break;
-        // features 112-207 (K-steps 7-12), accumulated
-        encode_cols<kTcHalfCols, 26>(a, kTcHalfCols, t, v, genc);
-        if (!mma_batch(g, t, tmem_d, a_base, kTcHalfCols * 128, w_base + 2 * param_off(0), 26 * 128, 7, 6, 64,
-                       true, mb, phase, &fail[g]))
-            break;
-        bool ok = true;
-        for (int l = 1; l <= 5 && ok; ++l) {
-            acc_to_a(tmem_row, a, t,
-                     keep ? reinterpret_cast<uint4*>(acts + (size_t)(l - 1) * ld * kHid + (size_t)row * kHid) : nullptr);
-            ok = mma_batch(g, t, tmem_d, a_base, 8 * 128, w_base + 2 * param_off(l), 8 * 128, 0, 4, l == 5 ? 16 : 64,
-                           false, mb, phase, &fail[g]);
-        }
-        if (!ok) break;
-        float o[16];
-        tmem_ld16(tmem_row, o);
-        if (row < n) {
-            out[3 * (size_t)row] = o[0];
-            out[3 * (size_t)row + 1] = o[1];
-            out[3 * (size_t)row + 2] = o[2];
-        }
-    }
-    tc_teardown(fail, tmem_base, err, mb, phase);
+// Contiguous bytes from global to shared memory (16-byte aligned, a multiple
+// of 16), counted on an mbarrier.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(mbar)
+                 : "memory");
 }
 
 // ---------------------------------------------------------------- inference on tcgen05
@@ -507,7 +307,7 @@ __global__ void __launch_bounds__(128 * kTcGroups, 1) k_mlp_fwd_tc(const float* 
 // 0.34 of the measured bf16 peak).
 // Waits are bounded; a warp whose wait gave up sets `fail`, which ends the
 // others' waits, and every tile's last commit is drained before the TMEM is
-// freed (see tc_teardown).
+// freed.
 constexpr int kInfGroups = 5;                   // warpgroups per CTA, at most
 constexpr uint32_t kInfCols = 96;               // TMEM columns per warpgroup: 64 accumulator, 32 operand
 
@@ -763,10 +563,7 @@ __global__ void __launch_bounds__(128 * kInfGroups, 1) k_mlp_infer_tc(const floa
     if (threadIdx.x == 0) {   // the weights, while the first tiles are encoded
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&wbar)), "r"(kTcWBytes)
                      : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         smem_u32(tc_smem)),
-                     "l"(wtc), "r"(kTcWBytes), "r"(smem_u32(&wbar))
-                     : "memory");
+        bulk_load(smem_u32(tc_smem), wtc, kTcWBytes, smem_u32(&wbar));
     }
     const uint32_t n = rows_of(cnt);
     const bool vec = ((uintptr_t)raw & 15u) == 0;
@@ -846,273 +643,491 @@ __global__ void __launch_bounds__(128 * kInfGroups, 1) k_mlp_infer_tc(const floa
     }
 }
 
-// ---------------------------------------------------------------- backward on tcgen05
-// k_mlp_bwd_tc: loss gradient (mean over the n rows and 3 channels), then
-// dOut of every layer back to the input (layer l at douts + l * ld * 64:
-// layers 0-4 [n][64], layer 5 [n][16]); accumulates the loss sum.  The tile
-// scheme of k_mlp_fwd_tc: thread t of a warpgroup owns row t, writes its
-// dOut_l into the A operand (K-major, no swizzle) and one thread issues
-// dAct_{l-1} = dOut_l * W_l with B = W_l^T from the transposed pack (N = 64
-// inputs, K = the layer's outputs: 16 for layer 5, else 64).  dOut_l is
-// dAct_l where layer l's stored activation is positive (ReLU), else 0.
-constexpr int kTcbWBytes = kTcbElems * 2;                       // 34,816
-constexpr int kTcbABytes = 128 / 8 * 8 * 128;                  // 16,384 (K = 64)
-constexpr int kTcbSmem = kTcbWBytes + kTcGroups * kTcbABytes;   // 100,352 at 4 warpgroups
+// ---------------------------------------------------------------- training forward and backward on tcgen05
+// k_mlp_train_tc: encoding, forward, loss gradient (mean over the n rows and 3
+// channels) and the way back through the layers, one 128-row tile at a time
+// per CTA of 256 threads, two CTAs per SM.  A training batch is a tile or two
+// per SM, so the kernel is one chain of 14 MMA batches and bound by its
+// latency: two threads share a row (warps w and w + 4 reach the same TMEM
+// lanes; the first half's warps write some columns of each operand, the second
+// half's the others), operands go straight to TMEM, the last of the eight
+// warps to finish its share issues the batch, both weight packs arrive by bulk
+// copies while the first rows are encoded, and each row's ReLU masks stay in
+// its threads' registers on the way back.  32,768 rows: 45 us as a
+// forward and a backward kernel with A in shared memory, 20 us now.
+// The weight gradients need the encoding ([n][208]), the five activations and
+// the six dOuts ([n][64], layer 5 [n][16]); they are stored in blocks of 8
+// rows x 8 features (128 bytes), which is how k_wgrad_tc's operands lie in
+// shared memory: feature block c of rows 8 b .. 8 b + 7 at block b * (features
+// / 8) + c.  Rows n .. up to the tile's end are stored too, with dOut = 0.
+constexpr int kTrThreads = 256, kTrWarps = kTrThreads / 32;
+constexpr int kTrSmem = kTcWBytes + kTcbWBytes;                // 96,256
+constexpr int kTrGrid = 296;                                   // CTAs, at most
+constexpr uint32_t kTrCols = 128;                              // TMEM columns: 64 accumulator, 32 operand
 
-__global__ void __launch_bounds__(128 * kTcGroups, 1) k_mlp_bwd_tc(const float* __restrict__ pred,
-                                                                   const float* __restrict__ target, NrcCount cnt,
-                                                                   uint32_t ld, const __nv_bfloat16* __restrict__ acts,
-                                                                   const __nv_bfloat16* __restrict__ wtcb,
-                                                                   __nv_bfloat16* __restrict__ douts,
-                                                                   float* __restrict__ loss_sum, uint32_t* err) {
-    extern __shared__ __align__(1024) uint8_t tc_smem[];
-    __shared__ __align__(8) uint64_t mbar[kTcGroups];
-    __shared__ int fail[kTcGroups];
-    __shared__ uint32_t tmem_base;
-    const int warp = threadIdx.x >> 5, g = warp >> 2, t = threadIdx.x & 127;
-    {
-        const uint4* src = reinterpret_cast<const uint4*>(wtcb);
-        uint4* dst = reinterpret_cast<uint4*>(tc_smem);
-        for (int k = threadIdx.x; k < kTcbWBytes / 16; k += blockDim.x) dst[k] = src[k];
+// What a thread keeps of its row between the parts of layer 0: the first half
+// the direction's and the normal's theta and the albedo, the second half
+// their phi and the last octave of axis 2.
+struct HalfRow {
+    float u0, u1, c0, c1, c2;
+};
+
+// Feature group KC of a row into its operand columns and its stored encoding.
+template <int KC>
+__device__ __forceinline__ void train_group(uint32_t tmem_a, uint4* genc, RowIn& v) {
+    const uint4 q = feature_group<KC>(v);
+    tmem_st4(tmem_a + 4 * (KC & 7), q.x, q.y, q.z, q.w);
+    genc[8 * KC] = q;
+}
+
+// A thread's share of layer-0 part `part` (groups 8 part .. 8 part + 7, at
+// most 25): axis 0 and the first octaves of axis 2 against axis 1 and the
+// rest of axis 2; the thetas' groups (9-12, 17-20) and the albedo against the
+// phis' (13-16, 21-24).
+__device__ __forceinline__ void encode_share(int part, int half, uint32_t tmem_a, uint4* genc,
+                                             const float* __restrict__ raw, uint32_t r, bool in_range, bool vec,
+                                             const Enc& e, HalfRow& k) {
+    RowIn v = {};
+    if (part == 0) {
+        float p[12] = {};
+        if (in_range) load_raw(raw, r, vec, p);
+        if (half == 0) {
+            k.u0 = row_theta(p[5]);
+            k.u1 = row_theta(p[8]);
+            k.c0 = p[9]; k.c1 = p[10]; k.c2 = p[11];
+            if (in_range) {
+                v.q[0] = (p[0] - e.x0) * e.sx;
+                v.q[2] = (p[2] - e.z0) * e.sz;
+            }
+            train_group<0>(tmem_a, genc, v);
+            train_group<1>(tmem_a, genc, v);
+            train_group<2>(tmem_a, genc, v);
+            train_group<6>(tmem_a, genc, v);
+        } else {
+            k.u0 = row_phi(p[3], p[4]);
+            k.u1 = row_phi(p[6], p[7]);
+            if (in_range) {
+                v.q[1] = (p[1] - e.y0) * e.sy;
+                v.q[2] = (p[2] - e.z0) * e.sz;
+            }
+            train_group<3>(tmem_a, genc, v);
+            train_group<4>(tmem_a, genc, v);
+            train_group<5>(tmem_a, genc, v);
+            feature_group<6>(v);        // octaves 0-3 of axis 2, for the chain
+            train_group<7>(tmem_a, genc, v);
+            k.c0 = v.ps[2];
+            k.c1 = v.pc[2];
+        }
+    } else if (half == 0) {
+        v.u[0] = k.u0;
+        v.u[2] = k.u1;
+        v.alb[0] = k.c0; v.alb[1] = k.c1; v.alb[2] = k.c2;
+        if (part == 1) {
+            train_group<9>(tmem_a, genc, v);
+            train_group<10>(tmem_a, genc, v);
+            train_group<11>(tmem_a, genc, v);
+            train_group<12>(tmem_a, genc, v);
+        } else if (part == 2) {
+            train_group<17>(tmem_a, genc, v);
+            train_group<18>(tmem_a, genc, v);
+            train_group<19>(tmem_a, genc, v);
+            train_group<20>(tmem_a, genc, v);
+        } else {
+            train_group<25>(tmem_a, genc, v);
+        }
+    } else {
+        v.u[1] = k.u0;
+        v.u[3] = k.u1;
+        if (part == 1) {
+            v.ps[2] = k.c0;
+            v.pc[2] = k.c1;
+            train_group<8>(tmem_a, genc, v);
+            train_group<13>(tmem_a, genc, v);
+            train_group<14>(tmem_a, genc, v);
+            train_group<15>(tmem_a, genc, v);
+        } else if (part == 2) {
+            train_group<16>(tmem_a, genc, v);
+            train_group<21>(tmem_a, genc, v);
+            train_group<22>(tmem_a, genc, v);
+            train_group<23>(tmem_a, genc, v);
+        } else {
+            train_group<24>(tmem_a, genc, v);
+        }
     }
-    tc_setup(mbar, fail, &tmem_base);
+}
+
+// 32 accumulator columns of a row.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < 32; ++k) v[k] = __uint_as_float(r[k]);
+}
+
+// Half a row's operand (32 features, 16 words): into its TMEM columns and, as
+// four 16-byte feature blocks, into memory.
+__device__ __forceinline__ void put_half(const uint32_t (&w)[16], uint32_t tmem_a, uint4* dst, bool operand) {
+    if (operand)
+        asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
+                tmem_a),
+            "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]),
+            "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
+            : "memory");
+#pragma unroll
+    for (int c = 0; c < 4; ++c) dst[8 * c] = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+}
+
+// Issues batch k of a tile: 0-8 the forward's (inf_issue), 9 dAct4 = dOut5 *
+// W5 (K = 16), 9 + i the same of layer 5 - i; then commits it.
+__device__ __forceinline__ void train_issue(int k, uint32_t tmem_d, uint32_t tmem_a, uint32_t w_base, uint32_t wb_base,
+                                            uint32_t mbar, uint32_t lane) {
+    if (k < 9) {
+        inf_issue(k, tmem_d, tmem_a, w_base, mbar, lane);
+        return;
+    }
+    constexpr uint32_t kLbo = (128u >> 4) << 16;
+    constexpr uint32_t kHi2 = (2u * 128u >> 4) | (1u << 14), kHi8 = (8u * 128u >> 4) | (1u << 14);
+    const int l = 14 - k;
+    const uint32_t b_lo = ((wb_base + 2u * (uint32_t)tcb_off(l)) >> 4) | kLbo;
+    constexpr uint32_t idesc = idesc_bf16(128, 64);
+    tc_fence_after();
+    if (lane == 0) {
+        if (l == 5) {
+            umma_ts(tmem_d, tmem_a, b_lo, kHi2, idesc, 0u);
+        } else {
+            umma_ts(tmem_d, tmem_a, b_lo, kHi8, idesc, 0u);
+            umma_ts(tmem_d, tmem_a + 8u, b_lo + 16u, kHi8, idesc, 1u);
+            umma_ts(tmem_d, tmem_a + 16u, b_lo + 32u, kHi8, idesc, 1u);
+            umma_ts(tmem_d, tmem_a + 24u, b_lo + 48u, kHi8, idesc, 1u);
+        }
+        umma_commit(mbar);
+    }
+}
+
+__global__ void __launch_bounds__(kTrThreads, 2) k_mlp_train_tc(const float* __restrict__ raw,
+                                                                const float* __restrict__ target, NrcCount cnt, Enc ec,
+                                                                const __nv_bfloat16* __restrict__ wtc,
+                                                                const __nv_bfloat16* __restrict__ wtcb, uint32_t ld,
+                                                                __nv_bfloat16* __restrict__ enc,
+                                                                __nv_bfloat16* __restrict__ acts,
+                                                                __nv_bfloat16* __restrict__ douts,
+                                                                float* __restrict__ loss_part, uint32_t* err) {
+    extern __shared__ __align__(1024) uint8_t tc_smem[];
+    __shared__ __align__(8) uint64_t mbar, wbar;   // the last batch is done; the weights are here
+    __shared__ uint32_t arrived, issued, tmem_base;
+    __shared__ int fail;
+    __shared__ float warp_loss[kTrWarps];
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);   // uniform, and known to be
+    const int half = warp >> 2;
+    const uint32_t lane = threadIdx.x & 31u, t = 32u * (warp & 3) + lane;    // t: row of the tile
+    if (threadIdx.x == 0) {
+        mbar_init(smem_u32(&mbar));
+        mbar_init(smem_u32(&wbar));
+        arrived = issued = 0;
+        fail = 0;
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
+                     "r"(kTrCols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&wbar)), "r"(kTrSmem)
+                     : "memory");
+        bulk_load(smem_u32(tc_smem), wtc, kTcWBytes, smem_u32(&wbar));
+        bulk_load(smem_u32(tc_smem + kTcWBytes), wtcb, kTcbWBytes, smem_u32(&wbar));
+    }
     const uint32_t n = rows_of(cnt);
     const float scale = n > 0 ? 1.0f / (3.0f * (float)n) : 0.0f;
-    const uint32_t tmem_d = tmem_base + 64u * g;
-    const uint32_t tmem_row = tmem_d + ((uint32_t)(32 * (warp & 3)) << 16);
-    uint8_t* a = tc_smem + kTcbWBytes + g * kTcbABytes;
-    const uint32_t a_base = smem_u32(a), w_base = smem_u32(tc_smem);
-    const uint32_t mb = smem_u32(&mbar[g]);
-    uint32_t phase = 0;
-    float loss = 0.0f;
+    const bool vec = ((uintptr_t)raw & 15u) == 0;
+    const uint32_t tmem_d = tmem_base, tmem_a = tmem_base + 64u;
+    const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;   // this warp's rows of them
+    const uint32_t mb = smem_u32(&mbar), w_base = smem_u32(tc_smem);
     const uint32_t tiles = (n + 127) / 128;
-    const uint32_t groups = blockDim.x >> 7;
-    for (uint32_t tile = blockIdx.x * groups + g; tile < tiles; tile += gridDim.x * groups) {
-        const uint32_t row = tile * 128 + t;
-        const bool ok = row < n;
-        // dL/dpred of the row's 3 channels -> dOut5 (K = 16: two core-matrix columns)
-        float d[3] = {0.0f, 0.0f, 0.0f};
-        if (ok) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float p = pred[3 * (size_t)row + c], y = target[3 * (size_t)row + c];
-                const float den = p * p + kLossEps, e = p - y;
-                loss += e * e / den;
-                d[c] = 2.0f * e / den * scale;
+    uint32_t parity = 0;
+    bool ok = true, weights_here = false;
+    float loss = 0.0f;
+    for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const uint32_t r = tile * 128u + t;
+        const bool in_range = r < n;
+        // 16-byte block of feature group 0 of this row, in arrays of F groups
+        auto block = [&](__nv_bfloat16* base, uint32_t F) {
+            return reinterpret_cast<uint4*>(base) + (size_t)(r >> 3) * F * 8u + (r & 7u);
+        };
+        HalfRow keep;
+        uint32_t mask[5];   // bit k: the low half of word k of this thread's activations is positive; k + 16: the high
+        for (int k = 0; k <= 14; ++k) {
+            if (k > 0) {
+                ok = warp_wait(mb, parity, &fail);
+                parity ^= 1u;
+                if (!ok) break;
             }
-        }
-        const uint4 q0 = make_uint4(pack(d[0], d[1]), pack(d[2], 0.0f), 0u, 0u), q1 = make_uint4(0u, 0u, 0u, 0u);
-        if (ok) {
-            uint4* g5 = reinterpret_cast<uint4*>(douts + (size_t)5 * ld * kHid + (size_t)row * kOut);
-            g5[0] = q0;
-            g5[1] = q1;
-        }
-        *reinterpret_cast<uint4*>(a + ((t >> 3) * 2) * 128 + (t & 7) * 16) = q0;
-        *reinterpret_cast<uint4*>(a + ((t >> 3) * 2 + 1) * 128 + (t & 7) * 16) = q1;
-        // dAct4 = dOut5 * W5
-        if (!mma_batch(g, t, tmem_d, a_base, 2 * 128, w_base + 2 * tcb_off(5), 2 * 128, 0, 1, 64, false, mb, phase,
-                       &fail[g]))
-            break;
-        bool go = true;
-        for (int l = 4; l >= 0 && go; --l) {
-            const uint4* gact = reinterpret_cast<const uint4*>(acts + (size_t)l * ld * kHid + (size_t)row * kHid);
-            uint4* gd = reinterpret_cast<uint4*>(douts + (size_t)l * ld * kHid + (size_t)row * kHid);
+            if (k < 4) {
+                encode_share(k, half, tmem_a + lanes, block(enc, kIn / 8), raw, r, in_range, vec, ec, keep);
+            } else if (k < 9) {
+                // layer k - 4's activation: accumulator -> bf16 -> ReLU (rounding is monotone)
+                float v[32];
+                tmem_ld32(tmem_d + lanes + 32u * half, v);
+                const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
+                uint32_t w[16], m = 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                float v[16];
-                tmem_ld16(tmem_row + 16 * q, v);
+                for (int q = 0; q < 16; ++q) {
+                    const __nv_bfloat162 b = __hmax2(__floats2bfloat162_rn(v[2 * q], v[2 * q + 1]), zero);
+                    w[q] = *reinterpret_cast<const uint32_t*>(&b);
+                    m |= (((w[q] & 0x7FFF7FFFu) + 0x7FFF7FFFu) & 0x80008000u) >> (15 - q);
+                }
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const uint4 m = ok ? gact[2 * q + h] : make_uint4(0u, 0u, 0u, 0u);
-                    const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
-                    uint32_t w[4];
+                for (int l = 0; l < 5; ++l)
+                    if (l == k - 4) mask[l] = m;
+                put_half(w, tmem_a + lanes + 16u * half, block(acts + (size_t)(k - 4) * ld * kHid, 8) + 32 * half, true);
+            } else if (k == 9) {
+                // prediction, loss and dL/dpred -> dOut5
+                if (half == 0) {
+                    float o[16];
+                    tmem_ld16(tmem_d + lanes, o);
+                    float d[3] = {0.0f, 0.0f, 0.0f};
+                    if (in_range) {
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float lo = lo_of(mw[k]) > 0.0f ? v[8 * h + 2 * k] : 0.0f;
-                        const float hi = hi_of(mw[k]) > 0.0f ? v[8 * h + 2 * k + 1] : 0.0f;
-                        w[k] = pack(lo, hi);
+                        for (int c = 0; c < 3; ++c) {
+                            const float p = o[c], y = target[3 * (size_t)r + c];
+                            const float den = p * p + kLossEps, e = p - y;
+                            loss += e * e / den;
+                            d[c] = 2.0f * e / den * scale;
+                        }
                     }
-                    const uint4 wv = make_uint4(w[0], w[1], w[2], w[3]);
-                    if (ok) gd[2 * q + h] = wv;
-                    *reinterpret_cast<uint4*>(a + ((t >> 3) * 8 + 2 * q + h) * 128 + (t & 7) * 16) = wv;
+                    const uint32_t w0 = pack(d[0], d[1]), w1 = pack(d[2], 0.0f);
+                    tmem_st4(tmem_a + lanes, w0, w1, 0u, 0u);
+                    tmem_st4(tmem_a + lanes + 4u, 0u, 0u, 0u, 0u);
+                    uint4* g5 = block(douts + (size_t)5 * ld * kHid, kOut / 8);
+                    g5[0] = make_uint4(w0, w1, 0u, 0u);
+                    g5[8] = make_uint4(0u, 0u, 0u, 0u);
+                }
+            } else {
+                // dOut_l = dAct_l where layer l's activation is positive
+                const int l = 14 - k;
+                float v[32];
+                tmem_ld32(tmem_d + lanes + 32u * half, v);
+                uint32_t w[16], m = 0;
+#pragma unroll
+                for (int q = 0; q < 5; ++q)
+                    if (q == l) m = mask[q];
+#pragma unroll
+                for (int q = 0; q < 16; ++q)
+                    w[q] = pack(v[2 * q], v[2 * q + 1]) & (((m >> q) & 0x00010001u) * 0xFFFFu);
+                put_half(w, tmem_a + lanes + 16u * half, block(douts + (size_t)l * ld * kHid, 8) + 32 * half, l > 0);
+                if (l == 0) {
+                    tc_fence_before();   // the next tile's batches overwrite the accumulator
+                    break;
                 }
             }
-            if (l == 0) break;
-            // dAct_{l-1} = dOut_l * W_l
-            go = mma_batch(g, t, tmem_d, a_base, 8 * 128, w_base + 2 * tcb_off(l), 8 * 128, 0, 4, 64, false, mb,
-                           phase, &fail[g]);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();     // accumulator reads and operand writes, ordered before the MMAs
+            __syncwarp();
+            uint32_t before = 0;
+            if (lane == 0)
+                asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
+                             : "=r"(before)
+                             : "r"(smem_u32(&arrived))
+                             : "memory");
+            before = __shfl_sync(0xFFFFFFFFu, before, 0);
+            if (before % kTrWarps == kTrWarps - 1) {   // the operand is complete
+                if (!weights_here) {
+                    uint32_t it = 0;
+                    while (!mbar_try_wait(smem_u32(&wbar), 0u) && ++it < kTcWaitCap) {}
+                    if (it >= kTcWaitCap) fail = 1;
+                    weights_here = true;
+                }
+                if (lane == 0) issued += 1;
+                train_issue(k, tmem_d, tmem_a, w_base, w_base + kTcWBytes, mb, lane);
+            }
+            __syncwarp();
         }
-        if (!go) break;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
-    if ((threadIdx.x & 31) == 0 && loss != 0.0f) atomicAdd(loss_sum, loss);
-    tc_teardown(fail, tmem_base, err, mb, phase);
+    if (lane == 0) warp_loss[warp] = loss;
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        tc_fence_after();
+        float sum = 0.0f;
+        for (int w = 0; w < kTrWarps; ++w) sum += warp_loss[w];
+        loss_part[blockIdx.x] = sum;
+        // the weights' copies and the last batch, before shared memory and
+        // TMEM are given back
+        uint32_t it = 0;
+        while (!mbar_try_wait(smem_u32(&wbar), 0u) && ++it < kTcDrainCap) {}
+        if (fail) {
+            it = 0;
+            while (issued && !mbar_try_wait(mb, (issued - 1u) & 1u) && ++it < kTcDrainCap) {}
+            atomicOr(err, kErrMlpTimeout);
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTrCols));
+    }
 }
 
 // ---------------------------------------------------------------- weight gradient on tcgen05
 // k_wgrad_tc: dW_l[o][i] = sum over rows r of dOut_l[r][o] * in_l[r][i], split
 // over the batch rows and the six layers: CTA (c, l) takes layer l's rows
 // [c * R, (c + 1) * R) and writes layer l's slice of partial c (k_reduce_adam
-// sums the partials).  One warpgroup per CTA; D = A * B with M = o, N = i
-// (208 or 64), K = rows, FP32 D in TMEM (256 or 64 columns).
-// Both operands are MN-major without swizzle, which is how the rows are stored
-// (features contiguous): a core matrix is 8 consecutive rows (K) x 8 features
-// (MN), 16 contiguous bytes per row, so staging is one 16-byte cp.async per
-// (row, 8 features), no transpose.
+// sums the partials, in the order of the chunks; chunks past the last row
+// write nothing).  D = A * B with
+// M = o, N = i (208 or 64), K = rows, FP32 D in TMEM (256 or 64 columns).
+// Both operands are MN-major without swizzle: a core matrix is 8 consecutive
+// rows (K) x 8 features (MN), 128 contiguous bytes, which is how
+// k_mlp_train_tc stores them:
 //   A (dOut_l^T): core matrix (o/8, r/8) at (r/8) * LBO_A + (o/8) * 128,
 //                 LBO_A = O * 16 (an 8-row group of all O outputs), SBO = 128;
 //   B (in_l):     core matrix (i/8, r/8) at (r/8) * LBO_B + (i/8) * 128,
 //                 LBO_B = I * 16, SBO = 128.
-// The MMA has M = 128 and the layer O = 64 or 16 real rows: the descriptor's
-// MN groups past O/8 read the bytes that follow (the next 8-row groups, and up
-// to kWgPad bytes past the tile, reserved), and the D rows they give are never
-// read.  Rows are staged kWgRows at a time into two buffers: one buffer's MMAs
-// run while the other fills.  Waits are bounded as in the forward kernel.
+// So 64 rows of an operand are one contiguous block, and a step is staged by
+// two bulk copies into a ring of kWgStages (A, then B behind it); one thread
+// keeps the ring full and issues the MMAs.  The MMA has M = 128 and the layer O
+// = 64 or 16 real rows: the descriptor's MN groups past O/8 read the bytes
+// that follow (the next 8-row groups, then B), and the D rows they give are
+// never read.  32,768 rows (60 MB of operands, 16 MB of partials): 28 us with
+// 16-byte copies by every thread from row-major arrays, 15.7 us now.  (Chunks of
+// 704 rows instead of 256, 47 partials instead of 128, took 12.6 us, but sum in
+// another order: after four Adam steps on the same batch the weights were 1e-4
+// from these.)  Waits are bounded as in the other kernels.
 constexpr int kWgRows = 64;                                   // rows per staging step (4 MMAs of K = 16)
-constexpr int kWgPad = 2048;                                  // bytes past an A tile its descriptor reads
-constexpr int kWgABytes = kWgRows / 8 * kHid * 16 + kWgPad;   // 10,240
-constexpr int kWgBBytes = kWgRows / 8 * kIn * 16;             // 26,624
-constexpr int kWgBuf = kWgABytes + kWgBBytes;                 // 36,864
-constexpr int kWgSmem = 2 * kWgBuf;                           // 73,728
+constexpr int kWgStages = 2;
+constexpr int kWgStage = kWgRows * (kHid + kIn) * 2;          // 34,816
+constexpr int kWgSmem = kWgStages * kWgStage;                 // 69,632: three CTAs per SM
 constexpr int kWgMinRows = 256;                               // rows per CTA, at least
+constexpr int kMaxPartials = 148;                             // row chunks (one FP32 partial each), at most
 
 __device__ __forceinline__ uint32_t idesc_bf16_mn(int m, int n) {
     return idesc_bf16(m, n) | (1u << 15) | (1u << 16);        // A and B MN-major
 }
 
-// Layer l's operand tiles for rows r0 .. r0 + kWgRows - 1 (zeros past n).
-__device__ __forceinline__ void wg_stage(uint8_t* buf, int l, uint32_t r0, uint32_t n, uint32_t ld,
-                                         const __nv_bfloat16* __restrict__ enc, const __nv_bfloat16* __restrict__ acts,
-                                         const __nv_bfloat16* __restrict__ douts) {
-    const int O = out_dim(l), I = in_dim(l);
-    const __nv_bfloat16* dsrc = douts + (size_t)l * ld * kHid;
-    const __nv_bfloat16* isrc = l == 0 ? enc : acts + (size_t)(l - 1) * ld * kHid;
-    const int oc = O / 8, ic = I / 8;
-    uint8_t* a = buf;
-    uint8_t* b = buf + kWgABytes;
-    for (int e = threadIdx.x; e < kWgRows * (oc + ic); e += blockDim.x) {
-        const int r = e / (oc + ic), c = e - r * (oc + ic);
-        const uint32_t row = r0 + (uint32_t)r;
-        const bool ok = row < n;
-        const size_t src_row = ok ? row : 0;
-        if (c < oc)
-            cp_async16(a + (r >> 3) * (O * 16) + c * 128 + (r & 7) * 16, dsrc + src_row * O + c * 8, ok);
-        else
-            cp_async16(b + (r >> 3) * (I * 16) + (c - oc) * 128 + (r & 7) * 16, isrc + src_row * I + (c - oc) * 8, ok);
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-
-// Bounded wait of the issuing thread on an mbarrier phase; false on a timeout.
-__device__ __forceinline__ bool wg_wait(uint32_t mbar, uint32_t parity) {
-    uint32_t it = 0;
-    while (!mbar_try_wait(mbar, parity) && ++it < kTcWaitCap) {}
-    return it < kTcWaitCap;
-}
-
 // Also advances the step counters (read by k_reduce_adam, which follows).
-__global__ void __launch_bounds__(128, 1) k_wgrad_tc(NrcCount cnt, uint32_t ld, uint32_t rows_per_cta,
+__global__ void __launch_bounds__(128, 3) k_wgrad_tc(NrcCount cnt, uint32_t ld, uint32_t rows_per_cta,
                                                      const __nv_bfloat16* __restrict__ enc,
                                                      const __nv_bfloat16* __restrict__ acts,
                                                      const __nv_bfloat16* __restrict__ douts,
                                                      float* __restrict__ partial, StepState* st, int do_step,
                                                      uint32_t* err) {
     extern __shared__ __align__(1024) uint8_t wg_smem[];
-    __shared__ __align__(8) uint64_t mbar[2];
-    __shared__ int fail[1];
+    __shared__ __align__(8) uint64_t full[kWgStages], done[kWgStages];
+    __shared__ int fail;
     __shared__ uint32_t tmem_base;
     const uint32_t n = rows_of(cnt);
     if (do_step && n > 0 && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {   // an empty batch takes no step
         st->step += 1;
         st->ema_steps += 1;
     }
+    const uint32_t row0 = blockIdx.x * rows_per_cta;
+    if (row0 >= n) return;
     const int t = threadIdx.x, warp = t >> 5;
     const int l = blockIdx.y;                        // this CTA's layer
+    const int O = out_dim(l), I = in_dim(l);
     const uint32_t cols = l == 0 ? 256u : 64u;       // TMEM columns: N = 208 or 64, a power of two
-    if (t < 2) mbar_init(smem_u32(&mbar[t]));
-    if (t == 0) fail[0] = 0;
+    const int steps = (int)((min(rows_per_cta, n - row0) + kWgRows - 1) / kWgRows);
+    if (t < kWgStages) {
+        mbar_init(smem_u32(&full[t]));
+        mbar_init(smem_u32(&done[t]));
+    }
+    if (t == 0) fail = 0;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
                      "r"(cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_d = tmem_base;
-    const uint32_t row0 = blockIdx.x * rows_per_cta;
-    const int steps = (int)(rows_per_cta / kWgRows);
-    float* part = partial + (size_t)blockIdx.x * kParams;
-    bool ok = true;
-    // the issuing thread's last commit (barrier and phase parity): a later
-    // commit covers every earlier MMA, so a drain waits on this one
-    uint32_t last_bar = 0, last_parity = 0;
-    wg_stage(wg_smem, l, row0, n, ld, enc, acts, douts);
-    for (int s = 0; s < steps && ok; ++s) {
-        const int b = s & 1;
-        uint8_t* buf = wg_smem + b * kWgBuf;
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        fence_proxy_async();        // this thread's copies, visible to the tensor core
+    if (t == 0) {
+        const uint8_t* a_src = reinterpret_cast<const uint8_t*>(douts + (size_t)l * ld * kHid) + (size_t)row0 * O * 2;
+        const uint8_t* b_src = reinterpret_cast<const uint8_t*>(l == 0 ? enc : acts + (size_t)(l - 1) * ld * kHid) +
+                               (size_t)row0 * I * 2;
+        const uint32_t a_bytes = kWgRows * O * 2, b_bytes = kWgRows * I * 2;
+        auto load = [&](int s) {
+            const int b = s % kWgStages;
+            const uint32_t dst = smem_u32(wg_smem + b * kWgStage), bar = smem_u32(&full[b]);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(a_bytes + b_bytes)
+                         : "memory");
+            bulk_load(dst, a_src + (size_t)s * a_bytes, a_bytes, bar);
+            bulk_load(dst + a_bytes, b_src + (size_t)s * b_bytes, b_bytes, bar);
+        };
+        auto wait = [&](uint64_t* bar, int s) {   // for step s's phase of its ring slot
+            uint32_t it = 0;
+            while (!mbar_try_wait(smem_u32(&bar[s % kWgStages]), (uint32_t)(s / kWgStages) & 1u) && ++it < kTcWaitCap) {}
+            return it < kTcWaitCap;
+        };
+        const uint32_t idesc = idesc_bf16_mn(128, I);
+        int loaded = 0, issued = 0;   // steps
+        bool ok = true;
+        for (; loaded < min(steps, kWgStages); ++loaded) load(loaded);
+        for (int s = 0; s < steps; ++s) {
+            if (!(ok = wait(full, s))) break;
+            tc_fence_after();
+            const uint32_t a0 = smem_u32(wg_smem + (s % kWgStages) * kWgStage), b0 = a0 + a_bytes;
+#pragma unroll
+            for (int ks = 0; ks < kWgRows / 16; ++ks)
+                umma(tmem_d, umma_desc(a0 + (uint32_t)(ks * 2 * O * 16), (uint32_t)(O * 16), 128u),
+                     umma_desc(b0 + (uint32_t)(ks * 2 * I * 16), (uint32_t)(I * 16), 128u), idesc,
+                     (s > 0 || ks > 0) ? 1u : 0u);
+            umma_commit(smem_u32(&done[s % kWgStages]));
+            issued = s + 1;
+            // the slot of step s - 1 takes step s - 1 + kWgStages once its MMAs are done
+            if (s >= 1 && loaded < steps) {
+                if (!(ok = wait(done, s - 1))) break;
+                load(loaded++);
+            }
+        }
+        if (ok) ok = wait(done, steps - 1);   // a commit covers every earlier MMA of the thread
+        if (!ok) {
+            // copies in flight and the last commit, before shared memory and TMEM are given back
+            uint32_t it = 0;
+            for (int s = max(0, loaded - kWgStages); s < loaded; ++s)
+                while (!mbar_try_wait(smem_u32(&full[s % kWgStages]), (uint32_t)(s / kWgStages) & 1u) && ++it < kTcDrainCap) {}
+            it = 0;
+            while (issued && !mbar_try_wait(smem_u32(&done[(issued - 1) % kWgStages]),
+                                            (uint32_t)((issued - 1) / kWgStages) & 1u) && ++it < kTcDrainCap) {}
+            fail = 1;
+            atomicOr(err, kErrMlpTimeout);
+        }
         tc_fence_before();
-        __syncthreads();
-        if (t == 0) {
-            tc_fence_after();
-            const int O = out_dim(l), I = in_dim(l);
-            const uint32_t a0 = smem_u32(buf), b0 = smem_u32(buf + kWgABytes);
-            const uint32_t idesc = idesc_bf16_mn(128, I);
-#pragma unroll 1
-            for (int ks = 0; ks < kWgRows / 16; ++ks) {
-                const uint64_t da = umma_desc(a0 + (uint32_t)(ks * 2 * O * 16), (uint32_t)(O * 16), 128u);
-                const uint64_t db = umma_desc(b0 + (uint32_t)(ks * 2 * I * 16), (uint32_t)(I * 16), 128u);
-                umma(tmem_d, da, db, idesc, (s > 0 || ks > 0) ? 1u : 0u);
-            }
-            umma_commit(smem_u32(&mbar[b]));
-            last_bar = smem_u32(&mbar[b]);
-            last_parity = (uint32_t)(s >> 1) & 1u;
-        }
-        // refill the other buffer with step s + 1 once step s - 1's MMAs (its
-        // last reader) are done
-        if (s + 1 < steps) {
-            if (s >= 1) {
-                if (t == 0 && !wg_wait(smem_u32(&mbar[b ^ 1]), ((s - 1) >> 1) & 1)) fail[0] = 1;
-                __syncthreads();
-                if (fail[0]) { ok = false; break; }
-            }
-            wg_stage(wg_smem + (b ^ 1) * kWgBuf, l, row0 + (uint32_t)((s + 1) * kWgRows), n, ld, enc, acts, douts);
-        }
-        if (s == steps - 1) {
-            // layer l complete: D rows o < O to this CTA's partial
-            if (t == 0 && !wg_wait(smem_u32(&mbar[b]), (s >> 1) & 1)) fail[0] = 1;
-            __syncthreads();
-            if (fail[0]) { ok = false; break; }
-            tc_fence_after();
-            const int O = out_dim(l), I = in_dim(l);
-            if (warp * 32 < O) {
-                float* dst = part + param_off(l) + (size_t)(warp * 32 + (t & 31)) * I;
-                const bool real = warp * 32 + (t & 31) < O;
-                for (int c0 = 0; c0 < I; c0 += 16) {
-                    float v[16];
-                    tmem_ld16(tmem_d + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-                    if (real) {
-                        float4* d4 = reinterpret_cast<float4*>(dst + c0);
-                        d4[0] = make_float4(v[0], v[1], v[2], v[3]);
-                        d4[1] = make_float4(v[4], v[5], v[6], v[7]);
-                        d4[2] = make_float4(v[8], v[9], v[10], v[11]);
-                        d4[3] = make_float4(v[12], v[13], v[14], v[15]);
-                    }
-                }
-            }
-        }
     }
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    // a wait that gave up: drain the last commit before the TMEM is freed
-    // (as tc_teardown does), then report
-    if (t == 0 && fail[0]) {
-        uint32_t it = 0;
-        while (!mbar_try_wait(last_bar, last_parity) && ++it < kTcDrainCap) {}
-        atomicOr(err, kErrMlpTimeout);
+    __syncthreads();
+    tc_fence_after();
+    // D rows o < O to this chunk's partial
+    if (!fail && warp * 32 < O) {
+        float* dst = partial + (size_t)blockIdx.x * kParams + param_off(l) + (size_t)(warp * 32 + (t & 31)) * I;
+        const bool real = warp * 32 + (t & 31) < O;
+        for (int c0 = 0; c0 < I; c0 += 16) {
+            float v[16];
+            tmem_ld16(tmem_d + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+            if (real) {
+                float4* d4 = reinterpret_cast<float4*>(dst + c0);
+                d4[0] = make_float4(v[0], v[1], v[2], v[3]);
+                d4[1] = make_float4(v[4], v[5], v[6], v[7]);
+                d4[2] = make_float4(v[8], v[9], v[10], v[11]);
+                d4[3] = make_float4(v[12], v[13], v[14], v[15]);
+            }
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -1137,17 +1152,45 @@ __device__ __forceinline__ void param_coords(int p, int& l, int& o, int& i) {
 // transposed, both in the tensor cores' canonical layout), and the inference
 // pack: with ema_a > 0, ema = ema_a * ema + (1 - ema_a) * w (ema
 // starts at 0) and the pack holds ema / (1 - ema_a^ema_steps), else w.
-__global__ void k_reduce_adam(const float* __restrict__ partial, int n_part, NrcCount cnt, float* __restrict__ grad,
-                              float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, AdamArgs ar,
-                              const StepState* __restrict__ st, int do_step, __nv_bfloat16* __restrict__ wtc,
-                              __nv_bfloat16* __restrict__ wtcb, float* __restrict__ ema,
-                              __nv_bfloat16* __restrict__ winf) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kParams) return;
+// A block takes kAdamParams parameters; its threads bring all their partials to
+// shared memory at once (one load at a time by the summing thread took 7.5 us
+// for 128 partials, 7.0 us now), and one thread each adds them in their
+// order.  One more block sums the loss.
+constexpr int kAdamParams = 64, kAdamThreads = 256;
+static_assert(kParams % kAdamParams == 0, "whole blocks");
+__global__ void __launch_bounds__(kAdamThreads)
+    k_reduce_adam(const float* __restrict__ partial, uint32_t rows_per_part, const float* __restrict__ loss_part,
+                  int n_loss, float* __restrict__ loss, NrcCount cnt, float* __restrict__ grad, float* __restrict__ w,
+                  float* __restrict__ m, float* __restrict__ v, AdamArgs ar, const StepState* __restrict__ st,
+                  int do_step, __nv_bfloat16* __restrict__ wtc, __nv_bfloat16* __restrict__ wtcb,
+                  float* __restrict__ ema, __nv_bfloat16* __restrict__ winf) {
+    __shared__ float s_part[kMaxPartials][kAdamParams];
+    if (blockIdx.x == kParams / kAdamParams) {
+        float sum = 0.0f;
+        for (int k = threadIdx.x; k < n_loss; k += kAdamThreads) sum += loss_part[k];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+        if ((threadIdx.x & 31) == 0) s_part[0][threadIdx.x >> 5] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < kAdamThreads / 32; ++k) sum += s_part[0][k];
+            *loss = sum;
+        }
+        return;
+    }
+    const int q = threadIdx.x % kAdamParams, p = blockIdx.x * kAdamParams + q;
+    const uint32_t n = rows_of(cnt);
+    const int n_part = (int)((n + rows_per_part - 1) / rows_per_part);   // the chunks that hold rows
+#pragma unroll 16
+    for (int k = threadIdx.x / kAdamParams; k < n_part; k += kAdamThreads / kAdamParams)
+        s_part[k][q] = __ldg(partial + (size_t)k * kParams + p);
+    __syncthreads();
+    if (threadIdx.x >= kAdamParams) return;
     float gsum = 0.0f;
-    for (int k = 0; k < n_part; ++k) gsum += partial[(size_t)k * kParams + p];
+#pragma unroll 8
+    for (int k = 0; k < n_part; ++k) gsum += s_part[k][q];
     grad[p] = gsum;
-    if (!do_step || rows_of(cnt) == 0) return;
+    if (!do_step || n == 0) return;
     const float step = (float)st->step;
     const float c1 = 1.0f - powf(ar.b1, step), c2 = 1.0f - powf(ar.b2, step);
     int l, o, i;
@@ -1204,7 +1247,7 @@ struct ilm_nrc {
     DeviceBuffer ema, winf;                      // moving average and its inference pack
     DeviceBuffer partial;                        // k_wgrad_tc partial sums
     DeviceBuffer err;                            // device error word (kErrMlpTimeout)
-    DeviceBuffer raw, enc, out, target, acts, douts, loss;
+    DeviceBuffer raw, enc, out, target, acts, douts, loss, loss_part;
     cudaStream_t stream = nullptr;
     ~ilm_nrc() {
         if (stream) cudaStreamDestroy(stream);
@@ -1212,24 +1255,6 @@ struct ilm_nrc {
 };
 
 namespace {
-
-// Launch shape of a tcgen05 MLP kernel for n rows: one 128-row tile per
-// warpgroup in flight, 4 warpgroups per CTA when the tiles fill the SMs that
-// way, else 2 or 1 so that they spread over more SMs (up to 2 CTAs per SM:
-// TMEM and shared memory allow it); each CTA stages the weights once and
-// strides over tiles.
-struct TcLaunch {
-    unsigned grid, threads;
-    size_t smem;
-};
-TcLaunch tc_launch(uint32_t n, int w_bytes, int a_bytes) {
-    const uint32_t tiles = (n + 127) / 128;
-    const uint32_t groups = tiles >= 4u * 148u ? 4u : (tiles >= 2u * 148u ? 2u : 1u);
-    uint32_t grid = (tiles + groups - 1) / groups;
-    const uint32_t cap = groups == 4 ? 148u : 296u;
-    grid = grid < 1 ? 1 : (grid > cap ? cap : grid);
-    return {grid, 128u * groups, (size_t)w_bytes + groups * (size_t)a_bytes};
-}
 
 Enc enc_params(const ilm_nrc* h) {
     const float* b = h->cfg.bound;
@@ -1249,71 +1274,62 @@ cudaError_t pack(ilm_nrc* h, cudaStream_t s) {
 uint32_t batch_cap(const NrcCount& c) { return c.batches > 1 ? (c.cap + c.batches - 1) / c.batches : c.cap; }
 
 cudaError_t reserve_train(ilm_nrc* h, uint32_t rows) {
+    const size_t ld = ((size_t)rows + 127) / 128 * 128;   // whole tiles
     cudaError_t e;
-    if ((e = h->enc.reserve((size_t)rows * kIn * 2)) != cudaSuccess) return e;
-    if ((e = h->out.reserve((size_t)rows * 3 * 4)) != cudaSuccess) return e;
-    if ((e = h->acts.reserve((size_t)rows * 5 * kHid * 2)) != cudaSuccess) return e;
-    return h->douts.reserve((size_t)rows * 6 * kHid * 2);
+    if ((e = h->enc.reserve(ld * kIn * 2)) != cudaSuccess) return e;
+    if ((e = h->acts.reserve(ld * 5 * kHid * 2)) != cudaSuccess) return e;
+    return h->douts.reserve(ld * 6 * kHid * 2);
 }
 
-// Training runs on the current weights and stores the encoding and the
-// activations (layer stride = the batch's row cap); inference runs on the
-// moving-average pack.
-cudaError_t forward(ilm_nrc* h, const float* raw, NrcCount cnt, bool train, float* out, cudaStream_t s) {
-    const uint32_t rows = batch_cap(cnt);
-    uint32_t* err = static_cast<uint32_t*>(h->err.ptr);
-    const TcLaunch L = tc_launch(rows, kTcWBytes, kTcABytes);
-    if (train)
-        k_mlp_fwd_tc<true><<<L.grid, L.threads, L.smem, s>>>(
-            raw, cnt, enc_params(h), static_cast<const __nv_bfloat16*>(h->wtc.ptr), out, err, rows,
-            static_cast<__nv_bfloat16*>(h->acts.ptr), static_cast<__nv_bfloat16*>(h->enc.ptr));
-    else {
-        // one CTA per SM, a warpgroup for every tile as long as there are SMs
-        // and warpgroups; TMEM columns are allocated in powers of two
-        const uint32_t tiles = std::max<uint32_t>(1, (rows + 127) / 128);
-        const uint32_t groups = std::min<uint32_t>(kInfGroups, (tiles + 147) / 148);
-        const uint32_t grid = std::min<uint32_t>(148, (tiles + groups - 1) / groups);
-        const uint32_t cols = groups == 1 ? 128u : (groups == 2 ? 256u : 512u);
-        k_mlp_infer_tc<<<grid, 128 * groups, kTcWBytes, s>>>(
-            raw, cnt, enc_params(h), static_cast<const __nv_bfloat16*>(h->winf.ptr), out, err, cols);
-    }
+// Network output with the inference weights (the moving-average pack).
+cudaError_t infer_rows(ilm_nrc* h, const float* raw, NrcCount cnt, float* out, cudaStream_t s) {
+    // one CTA per SM, a warpgroup for every tile as long as there are SMs and
+    // warpgroups; TMEM columns are allocated in powers of two
+    const uint32_t tiles = std::max<uint32_t>(1, (batch_cap(cnt) + 127) / 128);
+    const uint32_t groups = std::min<uint32_t>(kInfGroups, (tiles + 147) / 148);
+    const uint32_t grid = std::min<uint32_t>(148, (tiles + groups - 1) / groups);
+    const uint32_t cols = groups == 1 ? 128u : (groups == 2 ? 256u : 512u);
+    k_mlp_infer_tc<<<grid, 128 * groups, kTcWBytes, s>>>(raw, cnt, enc_params(h),
+                                                         static_cast<const __nv_bfloat16*>(h->winf.ptr), out,
+                                                         static_cast<uint32_t*>(h->err.ptr), cols);
     return cudaGetLastError();
 }
 
-// Loss gradient into h->grad (and the loss sum into h->loss, zeroed first);
-// with do_step, one Adam step.
+// Loss gradient of the current weights into h->grad and the loss sum into
+// h->loss; with do_step, one Adam step.
 cudaError_t train_rows(ilm_nrc* h, const float* raw, const float* target, NrcCount cnt, int do_step,
                        cudaStream_t s) {
     cudaError_t e;
-    const uint32_t cap = batch_cap(cnt);   // layer stride of acts / douts
+    const uint32_t cap = batch_cap(cnt);
     if ((e = reserve_train(h, cap)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(h->loss.ptr, 0, 4, s)) != cudaSuccess) return e;
-    float* pred = static_cast<float*>(h->out.ptr);
-    if ((e = forward(h, raw, cnt, true, pred, s)) != cudaSuccess) return e;
-    const __nv_bfloat16* acts = static_cast<const __nv_bfloat16*>(h->acts.ptr);
+    const uint32_t tiles = (cap + 127) / 128, ld = tiles * 128;   // ld: layer stride of acts / douts
+    const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(kTrGrid, tiles));
+    __nv_bfloat16* enc = static_cast<__nv_bfloat16*>(h->enc.ptr);
+    __nv_bfloat16* acts = static_cast<__nv_bfloat16*>(h->acts.ptr);
     __nv_bfloat16* douts = static_cast<__nv_bfloat16*>(h->douts.ptr);
-    const TcLaunch L = tc_launch(cap, kTcbWBytes, kTcbABytes);
-    k_mlp_bwd_tc<<<L.grid, L.threads, L.smem, s>>>(
-        pred, target, cnt, cap, acts, static_cast<const __nv_bfloat16*>(h->wtcb.ptr), douts,
-        static_cast<float*>(h->loss.ptr), static_cast<uint32_t*>(h->err.ptr));
+    float* loss_part = static_cast<float*>(h->loss_part.ptr);
+    uint32_t* err = static_cast<uint32_t*>(h->err.ptr);
+    k_mlp_train_tc<<<grid, kTrThreads, kTrSmem, s>>>(raw, target, cnt, enc_params(h),
+                                                     static_cast<const __nv_bfloat16*>(h->wtc.ptr),
+                                                     static_cast<const __nv_bfloat16*>(h->wtcb.ptr), ld, enc, acts, douts,
+                                                     loss_part, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    // split-K over the rows: kWgMinRows or more per CTA (a multiple of
-    // kWgRows), at most kMaxPartials CTAs
+    // row chunks of kWgMinRows or more (a multiple of kWgRows), at most kMaxPartials
     uint32_t per_cta = (cap + kMaxPartials - 1) / kMaxPartials;
     per_cta = std::max<uint32_t>(kWgMinRows, (per_cta + kWgRows - 1) / kWgRows * kWgRows);
-    const int n_part = (int)std::max<uint32_t>(1, (cap + per_cta - 1) / per_cta);
+    const uint32_t chunks = std::max<uint32_t>(1, (cap + per_cta - 1) / per_cta);
     StepState* st = static_cast<StepState*>(h->state.ptr);
-    k_wgrad_tc<<<dim3(n_part, kLayers), 128, kWgSmem, s>>>(cnt, cap, per_cta, static_cast<const __nv_bfloat16*>(h->enc.ptr), acts,
-                                            douts, static_cast<float*>(h->partial.ptr), st, do_step,
-                                            static_cast<uint32_t*>(h->err.ptr));
+    k_wgrad_tc<<<dim3(chunks, kLayers), 128, kWgSmem, s>>>(cnt, ld, per_cta, enc, acts, douts,
+                                                           static_cast<float*>(h->partial.ptr), st, do_step, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     AdamArgs ar{h->cfg.lr, h->cfg.beta1, h->cfg.beta2, h->cfg.eps,
                 h->cfg.ema > 0.0f && h->cfg.ema < 1.0f ? h->cfg.ema : 0.0f, h->cfg.weight_decay};
-    k_reduce_adam<<<(kParams + 255) / 256, 256, 0, s>>>(
-        static_cast<const float*>(h->partial.ptr), n_part, cnt, static_cast<float*>(h->grad.ptr),
-        static_cast<float*>(h->w.ptr), static_cast<float*>(h->m.ptr), static_cast<float*>(h->v.ptr), ar, st, do_step,
-        static_cast<__nv_bfloat16*>(h->wtc.ptr), static_cast<__nv_bfloat16*>(h->wtcb.ptr),
-        static_cast<float*>(h->ema.ptr), static_cast<__nv_bfloat16*>(h->winf.ptr));
+    k_reduce_adam<<<kParams / kAdamParams + 1, kAdamThreads, 0, s>>>(
+        static_cast<const float*>(h->partial.ptr), per_cta, loss_part, (int)grid, static_cast<float*>(h->loss.ptr), cnt,
+        static_cast<float*>(h->grad.ptr), static_cast<float*>(h->w.ptr), static_cast<float*>(h->m.ptr),
+        static_cast<float*>(h->v.ptr), ar, st, do_step, static_cast<__nv_bfloat16*>(h->wtc.ptr),
+        static_cast<__nv_bfloat16*>(h->wtcb.ptr), static_cast<float*>(h->ema.ptr),
+        static_cast<__nv_bfloat16*>(h->winf.ptr));
     return cudaGetLastError();
 }
 
@@ -1329,7 +1345,7 @@ cudaError_t take(DeviceBuffer& dst, const float* src, size_t bytes, cudaStream_t
 namespace ilm {
 
 cudaError_t nrc_infer_async(ilm_nrc* h, const float* raw, NrcCount n, float* out, cudaStream_t s) {
-    return forward(h, raw, n, false, out, s);
+    return infer_rows(h, raw, n, out, s);
 }
 
 cudaError_t nrc_train_async(ilm_nrc* h, const float* raw, const float* target, NrcCount n, cudaStream_t s) {
@@ -1363,6 +1379,7 @@ int32_t ilm_nrc_create(ilm_context* ctx, const ilm_nrc_config* cfg, ilm_nrc** ou
     if ((e = h->winf.reserve(kParams * 2)) != cudaSuccess) return cuda_fail(ctx, e, "nrc");
     if ((e = h->wtcb.reserve(kTcbElems * 2)) != cudaSuccess) return cuda_fail(ctx, e, "nrc");
     if ((e = h->loss.reserve(4)) != cudaSuccess) return cuda_fail(ctx, e, "nrc");
+    if ((e = h->loss_part.reserve(kTrGrid * 4)) != cudaSuccess) return cuda_fail(ctx, e, "nrc");
     if ((e = h->err.reserve(4)) != cudaSuccess) return cuda_fail(ctx, e, "nrc");
     cudaMemset(h->err.ptr, 0, 4);
     if ((e = h->state.reserve(sizeof(StepState))) != cudaSuccess) return cuda_fail(ctx, e, "nrc");
@@ -1386,8 +1403,7 @@ int32_t ilm_nrc_create(ilm_context* ctx, const ilm_nrc_config* cfg, ilm_nrc** ou
     cudaMemset(h->wtc.ptr, 0, kParams * 2);
     cudaMemset(h->winf.ptr, 0, kParams * 2);
     cudaMemset(h->wtcb.ptr, 0, kTcbElems * 2);
-    cudaFuncSetAttribute(k_mlp_fwd_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-    cudaFuncSetAttribute(k_mlp_bwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcbSmem);
+    cudaFuncSetAttribute(k_mlp_train_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem);
     cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
     cudaFuncSetAttribute(k_mlp_infer_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcWBytes);
     if ((e = pack(h.get(), h->stream)) != cudaSuccess) return cuda_fail(ctx, e, "nrc pack");
@@ -1437,7 +1453,7 @@ int32_t ilm_nrc_infer(ilm_context* ctx, ilm_nrc* h, const float* inputs, uint64_
         if ((e = h->out.reserve(n * 12)) != cudaSuccess) return cuda_fail(ctx, e, "nrc buffers");
         dst = static_cast<float*>(h->out.ptr);
     }
-    if ((e = forward(h, raw, NrcCount{nullptr, (uint32_t)n, 1, 0}, false, dst, s)) != cudaSuccess)
+    if ((e = infer_rows(h, raw, NrcCount{nullptr, (uint32_t)n, 1, 0}, dst, s)) != cudaSuccess)
         return cuda_fail(ctx, e, "nrc forward");
     if (!dev_out) {
         cudaMemcpyAsync(out, dst, n * 12, cudaMemcpyDeviceToHost, s);
