@@ -5,7 +5,6 @@
 #include "builder.h"
 
 #include <algorithm>
-#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -391,114 +390,18 @@ struct Entry {
     Box box;
 };
 
-// Which binary subtrees become the children of each wide node: the choice of
-// least expected traversal cost, by dynamic programming over the binary tree
-// (Ylitie, Karras and Laine, HPG 2017, section 3.1).  A wide node costs its
-// surface area, a leaf kPrimCost times its area per primitive.  F(n, k) is the
-// least cost of subtree n as at most k children of one wide node:
-//   F(n, 1) = min(a leaf, if it has at most kMaxLeafPrims primitives;
-//                 a wide node of its own: area + min_j F(left, j) + F(right, W - j))
-//   F(n, k) = min(F(n, k - 1), min_j F(left, j) + F(right, k - j)).
-// Opening the child of largest area until W were there (the rule before) left
-// 8-wide nodes 4.8 children full near the leaves; with this plan they hold
-// 7.6, and 1.3M triangles take 143K nodes instead of 348K.  Measured us,
-// before / after: a 1024 x 1024 render at 16 spp 36,000 / 33,900, eight
-// scenes batched 291 / 285, 2,000,003 shadow rays 183 / 181, 2,097,152
-// closest-hit ball rays 241 / 238.  kPrimCost from 0.4 to 5 moves these by
-// 1 to 5 %: below 1, leaves of two to four triangles stop a warp's node lanes
-// for longer, and the incoherent rays lose what the render gains.
-constexpr float kPrimCost = 1.5f;
-struct CollapsePlan {
-    static constexpr uint8_t kLeaf = 15;    // F(n, 1): a leaf
-    const std::vector<BinNode>& bin;
-    int W;
-    std::vector<uint32_t> first, count;     // primitives of each subtree
-    std::vector<uint64_t> choice;           // 4 bits per k: j of F(n, k); 0: as F(n, k - 1).  k = W + 1 in the
-                                            // top bits: j of the node's own split (k = 1)
-
-    CollapsePlan(const std::vector<BinNode>& b, int w) : bin(b), W(w) {
-        const size_t n = bin.size();
-        first.resize(n);
-        count.resize(n);
-        choice.resize(n);
-        std::vector<std::array<float, 9>> stack;
-        for (size_t i = n; i-- > 0;) {
-            const BinNode& nd = bin[i];
-            const float area = area_of(nd);
-            std::array<float, 9> f;
-            uint64_t ch = 0;
-            if (nd.n_prims) {
-                first[i] = (uint32_t)nd.offset;
-                count[i] = nd.n_prims;
-                f.fill(area * kPrimCost * (float)nd.n_prims);
-                ch = kLeaf << 4;
-            } else {
-                const size_t l = i + 1, r = (size_t)nd.offset;
-                first[i] = first[l];
-                count[i] = count[l] + count[r];
-                const std::array<float, 9> fl = stack.back();
-                stack.pop_back();
-                const std::array<float, 9> fr = stack.back();
-                stack.pop_back();
-                auto split = [&](int k, uint64_t& j_best) {
-                    float best = fl[1] + fr[k - 1];
-                    j_best = 1;
-                    for (int j = 2; j < k; ++j)
-                        if (fl[j] + fr[k - j] < best) { best = fl[j] + fr[k - j]; j_best = (uint64_t)j; }
-                    return best;
-                };
-                uint64_t j = 0;
-                f[1] = area + split(W, j);
-                ch |= j << 60;
-                if (count[i] <= kMaxLeafPrims) {
-                    const float leaf = area * kPrimCost * (float)count[i];
-                    if (leaf <= f[1]) { f[1] = leaf; ch |= (uint64_t)kLeaf << 4; }
-                }
-                for (int k = 2; k <= W; ++k) {
-                    const float s = split(k, j);
-                    if (s <= f[k - 1]) { f[k] = s; ch |= j << (4 * k); }
-                    else f[k] = f[k - 1];
-                }
-            }
-            choice[i] = ch;
-            stack.push_back(f);
-        }
-    }
-    static float area_of(const BinNode& n) {
-        const float x = n.bmax[0] - n.bmin[0], y = n.bmax[1] - n.bmin[1], z = n.bmax[2] - n.bmin[2];
-        return x * y + y * z + z * x;
-    }
-    bool leaf(uint32_t i) const { return ((choice[i] >> 4) & 15u) == kLeaf; }
-    // Subtree i as at most k children, appended to out.
-    void spread(uint32_t i, int k, std::vector<uint32_t>& out) const {
-        while (k > 1 && ((choice[i] >> (4 * k)) & 15u) == 0) --k;
-        if (k == 1 || bin[i].n_prims) { out.push_back(i); return; }
-        const int j = (int)((choice[i] >> (4 * k)) & 15u);
-        spread(i + 1, j, out);
-        spread((uint32_t)bin[i].offset, k - j, out);
-    }
-    // The children of subtree i's own wide node (i interior).
-    void children(uint32_t i, std::vector<uint32_t>& out) const {
-        const int j = (int)(choice[i] >> 60);
-        spread(i + 1, j, out);
-        spread((uint32_t)bin[i].offset, W - j, out);
-    }
-};
-
 struct Collapser {
     const std::vector<BinNode>& bin;
     const std::vector<BuildPrim>& prims;
     int W;
-    CollapsePlan plan{bin, W};
 
-    // Subtree i as a child: a leaf, or a wide node of its own.
     Entry from_bin(uint32_t i) const {
         const BinNode& n = bin[i];
         Entry e;
-        e.interior = !plan.leaf(i);
+        e.interior = n.n_prims == 0;
         e.bin = i;
-        e.start = e.interior ? 0 : plan.first[i];
-        e.count = e.interior ? 0 : plan.count[i];
+        e.start = e.interior ? 0 : (uint32_t)n.offset;
+        e.count = e.interior ? 0 : n.n_prims;
         for (int k = 0; k < 3; ++k) { e.box.mn[k] = n.bmin[k]; e.box.mx[k] = n.bmax[k]; }
         return e;
     }
@@ -513,18 +416,23 @@ struct Collapser {
         return e;
     }
     static bool expandable(const Entry& e) { return e.interior || e.count > kMaxLeafPrims; }
+    void split(const Entry& e, Entry out[2]) const {
+        if (e.interior) {
+            out[0] = from_bin(e.bin + 1);
+            out[1] = from_bin((uint32_t)bin[e.bin].offset);
+        } else {
+            uint32_t h = e.count / 2;
+            out[0] = range(e.start, h);
+            out[1] = range(e.start + h, e.count - h);
+        }
+    }
     std::vector<Entry> children_of(const Entry& e) const {
         std::vector<Entry> c;
         if (!expandable(e)) { c.push_back(e); return c; }
-        if (e.interior) {
-            std::vector<uint32_t> ids;
-            plan.children(e.bin, ids);
-            for (uint32_t i : ids) c.push_back(from_bin(i));
-            return c;
-        }
-        // a binary leaf of more primitives than a leaf child holds: halves,
-        // the largest first
-        c.push_back(e);
+        Entry s[2];
+        split(e, s);
+        c.push_back(s[0]);
+        c.push_back(s[1]);
         while ((int)c.size() < W) {
             int best = -1;
             float best_sa = -1.0f;
@@ -534,10 +442,9 @@ struct Collapser {
                     if (sa > best_sa) { best_sa = sa; best = (int)i; }
                 }
             if (best < 0) break;
-            const Entry b = c[best];
-            const uint32_t h = b.count / 2;
-            c[best] = range(b.start, h);
-            c.insert(c.begin() + best + 1, range(b.start + h, b.count - h));
+            split(c[best], s);
+            c[best] = s[0];
+            c.insert(c.begin() + best + 1, s[1]);
         }
         return c;
     }
