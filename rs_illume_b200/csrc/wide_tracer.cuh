@@ -1,10 +1,9 @@
 // Wide-BVH traversal state shared by the single-scene and batched kernels.
 //
 // Nodes are the compressed layout of layout.h: 8-bit child planes on a
-// per-node power-of-two grid, rounded outward at build time; a plane's
-// distance along the ray is one fma, and every test below is at least as
-// permissive as Bounds3::intersect_p on the exact child box
-// (geometry/bounds3.rs:284-318).
+// per-node power-of-two grid, dequantised with one fma each and rounded
+// outward at build time, so every test below is at least as permissive as
+// Bounds3::intersect_p on the exact child box (geometry/bounds3.rs:284-318).
 // Hit children are sorted by entry distance (sorting network on keys that
 // pack the distance's bits with the slot) and pushed far-to-near.
 #pragma once
@@ -16,128 +15,92 @@ template <int W> struct WideWords;
 template <> struct WideWords<8> { static constexpr int kWords = 5; };
 template <> struct WideWords<4> { static constexpr int kWords = 4; };
 
-// The float 2^15 + byte, formed by one byte permute that writes the byte into
-// bits 8-15 of 2^15, whose last place is 2^-8 (no integer-to-float
-// conversion: those issue on the narrow XU pipe, which 48 conversions per
-// node saturate).
-__device__ __forceinline__ float byte_float(uint32_t lo, uint32_t hi, int i) {
-    return __uint_as_float(__byte_perm(i < 4 ? lo : hi, 0x47000000u, ((uint32_t)(i & 3) << 4) | 0x7604u));
+// Byte i of a W-byte array split over 32-bit words lo (bytes 0-3) and hi (4-7).
+__device__ __forceinline__ uint32_t byte_of(uint32_t lo, uint32_t hi, int i) {
+    return __byte_perm(i < 4 ? lo : hi, 0u, (uint32_t)(i & 3) | 0x4440u);
 }
 
-// Largest magnitude of a reciprocal direction in the child tests: a zero (or
-// nearly zero) component keeps finite slab distances, so the sums below make
-// no NaN and an axis-parallel ray is still culled by that axis.
-constexpr float kMaxInv = 0x1p80f;
-__device__ __forceinline__ float clamp_inv(float i) { return fminf(fmaxf(i, -kMaxInv), kMaxInv); }
-
-// Child planes as distances along the ray: plane q of an axis lies at
-// grid start D + q s, so its distance (D + q s - o) / d is linear in q and
-// costs one fma on the byte's float, t = (2^15 + q) A + B with A = s / d and
-// B = (D - o) / d - 2^15 A.  The traversal is bound by the instructions it
-// issues, and forming the plane first took an fma, a subtract and a multiply
-// per plane: 157.8M warp instructions for 2,097,152 ball rays on 1.3M
-// triangles, 148.1M now with the entries below (255 to 241 us); 65,536 camera
-// rays on a 32,768-triangle soup 97 to 88 us.
-// The distances are approximate where the plane test was exact about its
-// plane, so both ends are moved outward:
-//  * the plane itself (D's rounding, and the host's check of the rounded
-//    plane) is off by at most 2^-23 |D| + 2^-16 s, and the sums by
-//    2^-24 (2^16 + 4 * 255) |A| < 2^-7 |A|: the margin 2^-22 |D| + 2^-6 s,
-//    as a distance, covers both twice;
-//  * what is left is at most 6 roundings of t itself at each end (1 / d among
-//    them): kWideRobust's 16 ulps cover the 12.
-// A child is thus hit whenever Bounds3::intersect_p hits its exact box.
-constexpr float kWideRobust = 0x1.00001p+0f;   // 1 + 2^-20
-struct AxisSlab {
-    float a, near_b, far_b;
-};
-__device__ __forceinline__ AxisSlab axis_slab(float origin, float scale, float o, float inv) {
-    const float start = fmaf(8388608.0f, scale, origin);   // the node's origin is biased by -2^23 scale
-    const float a = scale * inv;
-    const float b = fmaf(-32768.0f, a, (start - o) * inv);
-    const float margin = fmaf(fabsf(start), 0x1p-22f, scale * 0x1p-6f);
-    return {a, fmaf(-margin, fabsf(inv), b), fmaf(margin, fabsf(inv), b)};
+// The float 2^23 + byte, formed by one byte permute that writes the byte into
+// the low mantissa bits of 2^23 (no integer-to-float conversion: those issue
+// on the narrow XU pipe, which 48 conversions per node saturate).  Nodes
+// store their origin biased by -2^23 * scale, so fma(2^23 + q, scale, origin)
+// is the dequantised plane with no subtraction of the bias.
+__device__ __forceinline__ float byte_float(uint32_t lo, uint32_t hi, int i) {
+    return __uint_as_float(__byte_perm(i < 4 ? lo : hi, 0x4B000000u, (uint32_t)(i & 3) | 0x7650u));
 }
 
 // Decoded node, with near/far planes already swapped for the ray octant.
 template <int W>
 struct WideView {
-    AxisSlab ax, ay, az;
-    uint32_t valid[2];             // bit 7 of each child's byte: a child is there
-    uint32_t imask;                // interior children
-    uint32_t node_base, leaf_base; // entry of an interior / leaf child at offset 0
-    uint32_t off[2];               // per child byte: what to add to its base
+    float ox, oy, oz, sx, sy, sz;
+    uint32_t imask, child_base, prim_base;
+    uint32_t meta[2];
     uint32_t nq[3][2], fq[3][2];   // near / far quantised planes per axis
 };
 
-// Stack entries: bit 31 a leaf, bits 2-30 the node or the first primitive
-// record, bits 0-1 a leaf's record count - 1.
-__device__ __forceinline__ uint32_t entry_index(uint32_t e) { return (e & ~kLeafFlag) >> 2; }
-
 template <int W>
-__device__ __forceinline__ WideView<W> load_wide(const uint4* __restrict__ nodes, uint32_t idx, const RayIn& r,
-                                                 float ix, float iy, float iz) {
+__device__ __forceinline__ WideView<W> load_wide(const uint4* __restrict__ nodes, uint32_t idx, bool negx,
+                                                 bool negy, bool negz) {
     WideView<W> v;
     const uint4* p = nodes + (size_t)idx * WideWords<W>::kWords;
     uint4 w0 = __ldg(p), w1 = __ldg(p + 1), w2 = __ldg(p + 2), w3 = __ldg(p + 3);
-    uint32_t lo[3][2], hi[3][2], meta[2];
+    v.ox = __uint_as_float(w0.x); v.oy = __uint_as_float(w0.y); v.oz = __uint_as_float(w0.z);
+    v.sx = __uint_as_float((w0.w & 0xFFu) << 23);
+    v.sy = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23);
+    v.sz = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23);
+    v.imask = w0.w >> 24;
+    v.child_base = w1.x;
+    v.prim_base = w1.y;
+    uint32_t lo[3][2], hi[3][2];
     if (W == 8) {
         uint4 w4 = __ldg(p + 4);
-        meta[0] = w1.z; meta[1] = w1.w;
+        v.meta[0] = w1.z; v.meta[1] = w1.w;
         lo[0][0] = w2.x; lo[0][1] = w2.y; lo[1][0] = w2.z; lo[1][1] = w2.w;
         lo[2][0] = w3.x; lo[2][1] = w3.y; hi[0][0] = w3.z; hi[0][1] = w3.w;
         hi[1][0] = w4.x; hi[1][1] = w4.y; hi[2][0] = w4.z; hi[2][1] = w4.w;
     } else {
-        meta[0] = w1.z; meta[1] = 0;
+        v.meta[0] = w1.z; v.meta[1] = 0;
         lo[0][0] = w1.w; lo[1][0] = w2.x; lo[2][0] = w2.y; hi[0][0] = w2.z; hi[1][0] = w2.w;
         hi[2][0] = w3.x;
         lo[0][1] = lo[1][1] = lo[2][1] = hi[0][1] = hi[1][1] = hi[2][1] = 0;
     }
-    v.ax = axis_slab(__uint_as_float(w0.x), __uint_as_float((w0.w & 0xFFu) << 23), r.ox, ix);
-    v.ay = axis_slab(__uint_as_float(w0.y), __uint_as_float(((w0.w >> 8) & 0xFFu) << 23), r.oy, iy);
-    v.az = axis_slab(__uint_as_float(w0.z), __uint_as_float(((w0.w >> 16) & 0xFFu) << 23), r.oz, iz);
-    v.imask = w0.w >> 24;
-    v.node_base = w1.x << 2;
-    v.leaf_base = (w1.y << 2) | kLeafFlag;
-#pragma unroll
-    for (int h = 0; h < W / 4; ++h) {
-        // a child's byte is count << 5 | offset with a count of 1 to 4 (1 for
-        // an interior child); its entry adds offset << 2 | count - 1
-        const uint32_t m = meta[h];
-        v.valid[h] = (m + 0x60606060u) & 0x80808080u;
-        v.off[h] = ((m & 0x1F1F1F1Fu) << 2) | ((((m | 0x80808080u) - 0x20202020u) >> 5) & 0x03030303u);
-    }
-    const bool neg[3] = {ix < 0.0f, iy < 0.0f, iz < 0.0f};
+    bool neg[3] = {negx, negy, negz};
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
-        for (int h = 0; h < W / 4; ++h) {
+        for (int h = 0; h < 2; ++h) {
             v.nq[a][h] = neg[a] ? hi[a][h] : lo[a][h];
             v.fq[a][h] = neg[a] ? lo[a][h] : hi[a][h];
         }
     return v;
 }
 
-// Slab test of child i, with its entry distance clamped to the ray's start
-// (fmaxf / fminf skip a NaN slab, which can only widen the accepted set).
+// Slab test of child i (Bounds3::intersect_p semantics on the dequantised
+// box; fmaxf/fminf skip a NaN slab, which can only widen the accepted set).
 template <int W>
-__device__ __forceinline__ bool child_hit(const WideView<W>& v, int i, float tmax, float& tn_out) {
-    const float tnx = fmaf(byte_float(v.nq[0][0], v.nq[0][W / 4 - 1], i), v.ax.a, v.ax.near_b);
-    const float tny = fmaf(byte_float(v.nq[1][0], v.nq[1][W / 4 - 1], i), v.ay.a, v.ay.near_b);
-    const float tnz = fmaf(byte_float(v.nq[2][0], v.nq[2][W / 4 - 1], i), v.az.a, v.az.near_b);
-    const float tfx = fmaf(byte_float(v.fq[0][0], v.fq[0][W / 4 - 1], i), v.ax.a, v.ax.far_b);
-    const float tfy = fmaf(byte_float(v.fq[1][0], v.fq[1][W / 4 - 1], i), v.ay.a, v.ay.far_b);
-    const float tfz = fmaf(byte_float(v.fq[2][0], v.fq[2][W / 4 - 1], i), v.az.a, v.az.far_b);
-    const float tn = fmaxf(fmaxf(fmaxf(tnx, tny), tnz), 0.0f);
-    const float tf = fminf(fminf(tfx, tfy), tfz) * kWideRobust;
+__device__ __forceinline__ bool child_hit(const WideView<W>& v, int i, const RayIn& r, float ix, float iy,
+                                          float iz, float tmax, float& tn_out) {
+    uint32_t m = byte_of(v.meta[0], v.meta[1], i);
+    float nx = fmaf(byte_float(v.nq[0][0], v.nq[0][1], i), v.sx, v.ox);
+    float fx = fmaf(byte_float(v.fq[0][0], v.fq[0][1], i), v.sx, v.ox);
+    float ny = fmaf(byte_float(v.nq[1][0], v.nq[1][1], i), v.sy, v.oy);
+    float fy = fmaf(byte_float(v.fq[1][0], v.fq[1][1], i), v.sy, v.oy);
+    float nz = fmaf(byte_float(v.nq[2][0], v.nq[2][1], i), v.sz, v.oz);
+    float fz = fmaf(byte_float(v.fq[2][0], v.fq[2][1], i), v.sz, v.oz);
+    float tnx = __fmul_rn(__fsub_rn(nx, r.ox), ix), tfx = __fmul_rn(__fsub_rn(fx, r.ox), ix);
+    float tny = __fmul_rn(__fsub_rn(ny, r.oy), iy), tfy = __fmul_rn(__fsub_rn(fy, r.oy), iy);
+    float tnz = __fmul_rn(__fsub_rn(nz, r.oz), iz), tfz = __fmul_rn(__fsub_rn(fz, r.oz), iz);
+    float tn = fmaxf(fmaxf(tnx, tny), tnz);
+    float tf = __fmul_rn(fminf(fminf(tfx, tfy), tfz), kBoxRobust);
     tn_out = tn;
-    return (v.valid[i >> 2] & (0x80u << (8 * (i & 3)))) != 0u && tn <= tf && tn < tmax;
+    return m != 0u && tn <= tf && tn < tmax && tf > 0.0f;
 }
 
 template <int W>
 __device__ __forceinline__ uint32_t child_entry(const WideView<W>& v, uint32_t slot) {
-    const uint32_t o = __byte_perm(v.off[0], v.off[W / 4 - 1], slot) & 0xFFu;
-    return (((v.imask >> slot) & 1u) ? v.node_base : v.leaf_base) + o;
+    uint32_t m = byte_of(v.meta[0], v.meta[1], (int)slot);
+    if ((v.imask >> slot) & 1u) return v.child_base + (m & 31u);
+    return kLeafFlag | ((v.prim_base + (m & 31u)) << 3) | ((m >> 5) - 1u);
 }
 
 __device__ __forceinline__ void cswap(uint32_t& a, uint32_t& b) {
@@ -163,8 +126,8 @@ __device__ __forceinline__ void sort_keys(uint32_t* k) {
 }
 
 // A subtree handed to another lane that the donor's own pop would have culled
-// (no node or leaf entry has all bits set: that would be a leaf of 4 records
-// at 2^29 - 1; kd-tree node indices stay below 2^30).
+// (no node or leaf entry has all bits set: that would be a leaf of 8 records
+// at 2^28 - 1; kd-tree node indices stay below 2^30).
 constexpr uint32_t kNoEntry = 0xFFFFFFFFu;
 
 // Per-lane traversal state of one ray over 4- or 8-wide nodes: hit children
@@ -181,8 +144,8 @@ struct WideTracerSorted {
     using Entry = uint2;
     static constexpr int kDepth = kStack;
     RayIn ray;
-    float ix, iy, iz;              // reciprocal direction, clamped (clamp_inv)
-    bool tr_ready, occluded;
+    float ix, iy, iz;
+    bool negx, negy, negz, tr_ready, occluded;
     TriRay tr;
     float best_t, bu, bv;
     uint32_t best, status, cur, iter;
@@ -197,14 +160,17 @@ struct WideTracerSorted {
         best = ILM_MISS;
         occluded = false;
         status = 0;
-        ix = clamp_inv(__frcp_rn(r.dx)); iy = clamp_inv(__frcp_rn(r.dy)); iz = clamp_inv(__frcp_rn(r.dz));
+        ix = __frcp_rn(r.dx); iy = __frcp_rn(r.dy); iz = __frcp_rn(r.dz);   // == 1/d exactly
+        negx = ix < 0.0f; negy = iy < 0.0f; negz = iz < 0.0f;
         tr_ready = false;
         cur = 0; iter = 0; sp = 0;
     }
 
     // The root box test BVHAccel performs first (the root node's bounds are
     // the world bound).
-    __device__ __forceinline__ bool enters(const float* b) const { return root_enters(ray, b); }
+    __device__ __forceinline__ bool enters(const float* b) const {
+        return box_intersect_p(b[0], b[1], b[2], b[3], b[4], b[5], ray, ix, iy, iz, negx, negy, negz, ray.tmax);
+    }
 
     // Starts on subtree `node` of a ray another lane is tracing, with that
     // lane's reciprocal directions and `bound` (its best distance so far) as
@@ -212,6 +178,7 @@ struct WideTracerSorted {
     __device__ __forceinline__ void adopt(const RayIn& r, float rx, float ry, float rz, float bound, uint32_t node) {
         ray = r;
         ix = rx; iy = ry; iz = rz;
+        negx = ix < 0.0f; negy = iy < 0.0f; negz = iz < 0.0f;
         best_t = bound; bu = 0.0f; bv = 0.0f;
         best = ILM_MISS;
         occluded = false;
@@ -259,14 +226,14 @@ struct WideTracerSorted {
 
     // Interior node `cur`: true when the traversal continues into a child.
     __device__ __forceinline__ bool node(const uint4* __restrict__ nodes) {
-        const WideView<W> nv = load_wide<W>(nodes, cur >> 2, ray, ix, iy, iz);
+        WideView<W> nv = load_wide<W>(nodes, cur, negx, negy, negz);
         float lim = kAny ? ray.tmax : best_t;
         if (kAny) {
             uint32_t first = 0xFFFFFFFFu;
 #pragma unroll
             for (int c = 0; c < W; ++c) {
                 float tn;
-                if (child_hit<W>(nv, c, lim, tn)) {
+                if (child_hit<W>(nv, c, ray, ix, iy, iz, lim, tn)) {
                     uint32_t e = child_entry<W>(nv, (uint32_t)c);
                     if (first == 0xFFFFFFFFu) first = e;
                     else if (sp < kStack) push(make_uint2(e, 0u));
@@ -281,8 +248,8 @@ struct WideTracerSorted {
 #pragma unroll
         for (int c = 0; c < W; ++c) {
             float tn;
-            bool h = child_hit<W>(nv, c, lim, tn);
-            keys[c] = h ? ((__float_as_uint(tn) & ~7u) | (uint32_t)c) : 0xFFFFFFFFu;
+            bool h = child_hit<W>(nv, c, ray, ix, iy, iz, lim, tn);
+            keys[c] = h ? ((__float_as_uint(fmaxf(tn, 0.0f)) & ~7u) | (uint32_t)c) : 0xFFFFFFFFu;
             nhit += h ? 1 : 0;
         }
         if (nhit == 0) return false;
@@ -296,7 +263,7 @@ struct WideTracerSorted {
     }
 
     __device__ __forceinline__ void leaf(const PrimRec* __restrict__ prims, const SphereRec* __restrict__ spheres) {
-        const uint32_t start = entry_index(cur), cnt = (cur & 3u) + 1u;
+        uint32_t start = (cur & ~kLeafFlag) >> 3, cnt = (cur & 7u) + 1u;
         for (uint32_t k = 0; k < cnt; ++k) {
             float t, u, v;
             uint32_t pid;
