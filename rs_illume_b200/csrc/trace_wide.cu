@@ -43,9 +43,9 @@ __global__ void __launch_bounds__(128) k_trace_wide(TraceArgs a) {
 // subtrees of the warp's rays, so fewer rays a warp shorten the longest ray's
 // chain of steps as long as the warps fit; beyond one wave they queue.
 // Measured us at 32 / 16 / chosen, camera rays on a 32,768-triangle soup:
-// 1,000 rays 79 / 55 / 29 (1 a warp), 10,000 94 / 64 / 41 (4), 33,000
-// 99 / 75 / 70 (8), and at half the chosen number 57 (10,000) and 91 (33,000);
-// incoherent rays gain 0 to 20 %.
+// 1,000 rays 84 / 59 / 31 (1 a warp), 10,000 104 / 70 / 43 (4), 33,000
+// 109 / 80 / 76 (8), and at a quarter of the chosen number 62 (10,000) and 98
+// (33,000); incoherent rays gain 0 to 30 %.
 __host__ __device__ __forceinline__ uint32_t rays_per_warp(uint64_t n, uint64_t threads) {
     uint32_t r = 1;
     while (r < 32u && n * 32u > threads * r) r *= 2u;
@@ -269,8 +269,8 @@ cudaError_t launch_persistent(const TraceArgs& t, cudaStream_t s) {
 
 // Persistent launch of either refill.  Accels of triangles alone always run
 // the kernel built for kOccupancyBlocks resident blocks per SM: its state fits
-// 72 registers without spills, and left to itself the compiler takes 117 to
-// 127 (4 blocks): 2,000,003 shadow rays on 1.3M triangles 183 against 220 us.
+// 72 registers without spills, and left to itself the compiler takes 80 to 90
+// (5 blocks): 2,000,003 shadow rays on 1.3M triangles 189 against 227 us.
 // With analytic shapes in the leaf loop that build spills 200 to 250 bytes,
 // and the caller's flag decides.
 constexpr int kOccupancyBlocks = 7;
