@@ -289,34 +289,41 @@ __global__ void k_pt_camera(PtArgs a, unsigned long long p0, uint32_t count) {
     if (kNrc) a.spread[0][k] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(tw));
 }
 
+// A path's vertex in phases, each of which ends where the warp appends to one
+// queue, so that a phase's ray is written before the next one's is made:
+// holding all of them to the end took 124 to 162 registers (two blocks per
+// SM).  The stage streams about 140 bytes a path in and 50 to 150 out, but is
+// bound by issue and the latency of hit -> triangle -> material -> light, so
+// three blocks per SM pay for the 50 to 100 bytes they spill: shading of a
+// 1024 x 1024 render at 16 spp 5.17 ms before, 4.35 now (4.65 at four blocks),
+// of four cache frames 1.39 and 0.82.  (Appending once per block instead made
+// the queues' order cost the traversal 0.6 ms of the render.)
+constexpr int kShadeBlock = 256;
 template <bool kNrc>
-__global__ void __launch_bounds__(256) k_pt_shade(PtArgs a, int cur) {
+__global__ void __launch_bounds__(kShadeBlock, 3) k_pt_shade(PtArgs a, int cur) {
     const uint32_t n = (uint32_t)a.counts[cur];
     const uint32_t depth = (uint32_t)a.counts[kDepth];
     const int nxt = cur ^ 1;
     const uint32_t stride = gridDim.x * blockDim.x;
     // every lane of a warp runs the same number of iterations (warp_append needs the whole warp)
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        uint32_t i = base + threadIdx.x;
-        bool valid = i < n;
-        bool cont = false, push_l = false, push_b = false, query = false;
-        float3 o_l, d_l, o_b, d_b, o_c, d_c;
-        float tm_l = 0.0f, tm_b = 0.0f;
-        float3 c_l = make_float3(0, 0, 0), c_b = make_float3(0, 0, 0);
-        float4 beta_out = make_float4(0, 0, 0, 0), spread_next = make_float4(0, 0, 0, 0);
-        uint2 rng_out = make_uint2(0, 0);
+        const uint32_t i = base + threadIdx.x;
+        // the vertex
+        bool live = false, query = false;
         uint32_t id = 0, fid = 0, tw = kNone;
-        float3 q_p, q_wo, q_n, q_alb, q_beta;
-        if (valid) {
+        float3 beta, p, perr, nrm, albedo;
+        float wo_z = 0.0f;
+        float4 sp = make_float4(0, 0, 0, 0);
+        Pcg32 rng;
+        if (i < n) {
             float4 b4 = a.beta[cur][i];
-            float3 beta = f3(b4);
+            beta = f3(b4);
             fid = __float_as_uint(b4.w);
             id = a.pid[cur][i];
             uint2 rs = a.rng[cur][i];
-            Pcg32 rng;
             rng.inc = (path_seq(a.seed, id) << 1u) | 1u;
             rng.state = (uint64_t)rs.x | ((uint64_t)rs.y << 32);
-            float4 sp = kNrc ? a.spread[cur][i] : make_float4(0, 0, 0, 0);
+            if (kNrc) sp = a.spread[cur][i];
             if (kNrc) tw = __float_as_uint(sp.w);
             ilm_hit h = a.hits[i];
             const float4* rp = reinterpret_cast<const float4*>(a.rays[cur] + i);
@@ -328,16 +335,16 @@ __global__ void __launch_bounds__(256) k_pt_shade(PtArgs a, int cur) {
                 uint32_t m = __float_as_uint(t0.w);
                 float3 p0 = f3(t0), p1 = f3(t1), p2 = f3(t2);
                 float b1 = h.u, b2 = h.v, b0 = 1.0f - b1 - b2;
-                float3 p = p0 * b0 + p1 * b1 + p2 * b2;
-                float3 perr = (abs3(p0 * b0) + abs3(p1 * b1) + abs3(p2 * b2)) * 0x1.c0000cp-22f;   // gamma(7)
-                float3 nrm = normalize3(cross3(p0 - p2, p1 - p2));
+                p = p0 * b0 + p1 * b1 + p2 * b2;
+                perr = (abs3(p0 * b0) + abs3(p1 * b1) + abs3(p2 * b2)) * 0x1.c0000cp-22f;   // gamma(7)
+                nrm = normalize3(cross3(p0 - p2, p1 - p2));
                 float3 wo = make_float3(-r1.x, -r1.y, -r1.z);
-                float3 albedo = f3(a.mat[2 * m]);
+                albedo = f3(a.mat[2 * m]);
                 if (depth == 0) {
                     float3 le = f3(a.mat[2 * m + 1]);
                     if (dot3(nrm, wo) > 0.0f) film_add(a, fid, beta * le);
                 }
-                float wo_z = dot3(wo, nrm);
+                wo_z = dot3(wo, nrm);
                 bool cache_here = false;
                 if (kNrc) {
                     float cosv = fmaxf(fabsf(wo_z), 1e-6f);
@@ -363,11 +370,7 @@ __global__ void __launch_bounds__(256) k_pt_shade(PtArgs a, int cur) {
                         tw = (tw & kSlotMask) | (left << 24);
                     }
                     const uint32_t slot = tw == kNone ? kNone : tw & kSlotMask;
-                    const bool record = slot != kNone && !cache_here;
-                    if (cache_here || record) {
-                        q_p = p; q_wo = wo; q_n = nrm; q_alb = albedo; q_beta = beta;
-                    }
-                    if (record) {
+                    if (slot != kNone && !cache_here) {
                         float* rec = a.t_rec + ((size_t)slot * a.max_depth + depth) * kRec;
                         float in[12] = {p.x, p.y, p.z, wo.x, wo.y, wo.z, nrm.x, nrm.y, nrm.z,
                                         albedo.x, albedo.y, albedo.z};
@@ -381,131 +384,151 @@ __global__ void __launch_bounds__(256) k_pt_shade(PtArgs a, int cur) {
                     }
                     query = cache_here;
                 }
-                if (!cache_here) {
-                    float3 ss, ts;
-                    frame(nrm, ss, ts);
-                    float u_sel = rng.uniform_float();
-                    float ul0 = rng.uniform_float(), ul1 = rng.uniform_float();
-                    float us0 = rng.uniform_float(), us1 = rng.uniform_float();
-                    // a black BSDF (f = 0) casts no visibility rays and ends the path
-                    const bool black = albedo.x == 0.0f && albedo.y == 0.0f && albedo.z == 0.0f;
-                    if (a.n_lights > 0 && wo_z != 0.0f && !black) {
-                        uint32_t k = min((uint32_t)(u_sel * (float)a.n_lights), a.n_lights - 1u);
-                        uint32_t lp_id = a.lights[k];
-                        float4 lg = a.light_geo[k];
-                        float3 nl = f3(lg);
-                        float area = lg.w;
-                        float3 q0 = f3(a.tri[3 * lp_id]), q1 = f3(a.tri[3 * lp_id + 1]), q2 = f3(a.tri[3 * lp_id + 2]);
-                        float3 le = f3(a.mat[2 * __float_as_uint(a.tri[3 * lp_id].w) + 1]);
-                        float nlf = (float)a.n_lights;
-                        // light sample (uniform_sample_triangle, sampling.rs:264-267)
-                        float su = sqrtf(ul0);
-                        float c0 = 1.0f - su, c1 = ul1 * su, c2 = 1.0f - c0 - c1;
-                        float3 pl = q0 * c0 + q1 * c1 + q2 * c2;
-                        float3 pl_err = (abs3(q0 * c0) + abs3(q1 * c1) + abs3(q2 * c2)) * 0x1.80000ap-22f;   // gamma(6)
-                        float3 wi = pl - p;
-                        float d2 = dot3(wi, wi);
-                        if (d2 > 0.0f) {
-                            wi = wi * rsqrtf(d2);
-                            float cl = dot3(nl, wi * -1.0f);
-                            float light_pdf = d2 / (fabsf(cl) * area);
-                            float wi_z = dot3(wi, nrm);
-                            bool reflect = wi_z * wo_z > 0.0f;
-                            if (cl > 0.0f && isfinite(light_pdf) && light_pdf > 0.0f && reflect) {
-                                float scat_pdf = fabsf(wi_z) * (1.0f / kPiF);
-                                float w = power_heuristic(light_pdf, scat_pdf);
-                                c_l = beta * albedo * le * ((1.0f / kPiF) * fabsf(wi_z) * w / light_pdf * nlf);
-                                o_l = offset_origin(p, perr, nrm, pl - p);
-                                float3 tgt = offset_origin(pl, pl_err, nl, o_l - pl);
-                                d_l = tgt - o_l;
-                                tm_l = 1.0f - 0.0001f;
-                                push_l = true;
-                            }
-                        }
-                        // BSDF sample with MIS
-                        float3 wl = cosine_hemisphere(us0, us1);
-                        if (wo_z < 0.0f) wl.z = -wl.z;
-                        float3 wb = ss * wl.x + ts * wl.y + nrm * wl.z;
-                        float scat_pdf = fabsf(wl.z) * (1.0f / kPiF);
-                        float wb_z = dot3(wb, nrm);
-                        if (scat_pdf > 0.0f && wb_z * wo_z > 0.0f) {
-                            float3 o = offset_origin(p, perr, nrm, wb);
-                            TriRay tr = make_tri_ray(o.x, o.y, o.z, wb.x, wb.y, wb.z);
-                            float tl, lb1, lb2;
-                            if (triangle_test(tr, q0, q1, q2, INFINITY, tl, lb1, lb2)) {
-                                float3 pli = q0 * (1.0f - lb1 - lb2) + q1 * lb1 + q2 * lb2;
-                                float3 dv = pli - p;
-                                float lpdf = dot3(dv, dv) / (fabsf(dot3(nl, wb)) * area);
-                                if (isfinite(lpdf) && lpdf > 0.0f && dot3(nl, wb) < 0.0f) {
-                                    float w = power_heuristic(scat_pdf, lpdf);
-                                    c_b = beta * albedo * le * ((1.0f / kPiF) * fabsf(wb_z) * w / scat_pdf * nlf);
-                                    o_b = o;
-                                    d_b = wb;
-                                    tm_b = tl * (1.0f - 0.0001f);
-                                    push_b = true;
-                                }
-                            }
-                        }
-                    }
-                    // continuation
-                    float u0 = rng.uniform_float(), u1 = rng.uniform_float();
-                    float urr = rng.uniform_float();
-                    float3 wl = cosine_hemisphere(u0, u1);
-                    if (wo_z < 0.0f) wl.z = -wl.z;
-                    float3 wi = ss * wl.x + ts * wl.y + nrm * wl.z;
-                    float pdf = fabsf(wl.z) * (1.0f / kPiF);
+                live = !cache_here;
+            }
+        }
+        if (kNrc) {
+            const uint32_t sq = warp_append(&a.counts[kQueries], query);
+            if (query && sq < a.q_cap) {
+                const float4* rp = reinterpret_cast<const float4*>(a.rays[cur] + i);
+                const float4 r1 = rp[1];
+                float* qi = a.q_in + 12 * (size_t)sq;
+                float in[12] = {p.x, p.y, p.z, -r1.x, -r1.y, -r1.z, nrm.x, nrm.y, nrm.z,
+                                albedo.x, albedo.y, albedo.z};
+#pragma unroll
+                for (int q = 0; q < 12; ++q) qi[q] = in[q];
+                a.q_beta[sq] = make_float4(beta.x, beta.y, beta.z, __uint_as_float(fid));
+                a.q_train[sq] = make_uint2(tw == kNone ? kNone : tw & kSlotMask, depth);
+            }
+        }
+        // the light sample
+        float3 ss, ts;
+        float us0 = 0.0f, us1 = 0.0f;
+        uint32_t lk = kNone;         // the chosen light
+        bool black = true, push = false;
+        float3 o_s, d_s, c_s;
+        float tm_s = 0.0f;
+        if (live) {
+            frame(nrm, ss, ts);
+            float u_sel = rng.uniform_float();
+            float ul0 = rng.uniform_float(), ul1 = rng.uniform_float();
+            us0 = rng.uniform_float();
+            us1 = rng.uniform_float();
+            // a black BSDF (f = 0) casts no visibility rays and ends the path
+            black = albedo.x == 0.0f && albedo.y == 0.0f && albedo.z == 0.0f;
+            if (a.n_lights > 0 && wo_z != 0.0f && !black) {
+                lk = min((uint32_t)(u_sel * (float)a.n_lights), a.n_lights - 1u);
+                const uint32_t lp_id = a.lights[lk];
+                float4 lg = a.light_geo[lk];
+                float3 nl = f3(lg);
+                float area = lg.w;
+                float3 q0 = f3(a.tri[3 * lp_id]), q1 = f3(a.tri[3 * lp_id + 1]), q2 = f3(a.tri[3 * lp_id + 2]);
+                float3 le = f3(a.mat[2 * __float_as_uint(a.tri[3 * lp_id].w) + 1]);
+                float nlf = (float)a.n_lights;
+                // light sample (uniform_sample_triangle, sampling.rs:264-267)
+                float su = sqrtf(ul0);
+                float c0 = 1.0f - su, c1 = ul1 * su, c2 = 1.0f - c0 - c1;
+                float3 pl = q0 * c0 + q1 * c1 + q2 * c2;
+                float3 pl_err = (abs3(q0 * c0) + abs3(q1 * c1) + abs3(q2 * c2)) * 0x1.80000ap-22f;   // gamma(6)
+                float3 wi = pl - p;
+                float d2 = dot3(wi, wi);
+                if (d2 > 0.0f) {
+                    wi = wi * rsqrtf(d2);
+                    float cl = dot3(nl, wi * -1.0f);
+                    float light_pdf = d2 / (fabsf(cl) * area);
                     float wi_z = dot3(wi, nrm);
-                    if (!black && wo_z != 0.0f && pdf > 0.0f && wi_z * wo_z > 0.0f) {
-                        float3 nb = beta * albedo * ((1.0f / kPiF) * fabsf(wi_z) / pdf);
-                        bool alive = true;
-                        if (depth >= a.rr_depth) {
-                            float q = fmaxf(0.05f, 1.0f - max3c(nb));
-                            if (urr < q) alive = false;
-                            else nb = nb * (1.0f / (1.0f - q));
-                        }
-                        if (alive && depth + 1 < a.max_depth) {
-                            o_c = offset_origin(p, perr, nrm, wi);
-                            d_c = wi;
-                            beta_out = make_float4(nb.x, nb.y, nb.z, __uint_as_float(fid));
-                            rng_out = make_uint2((uint32_t)rng.state, (uint32_t)(rng.state >> 32));
-                            spread_next = make_float4(sp.x, sp.y, pdf, __uint_as_float(tw));
-                            cont = true;
-                        }
+                    bool reflect = wi_z * wo_z > 0.0f;
+                    if (cl > 0.0f && isfinite(light_pdf) && light_pdf > 0.0f && reflect) {
+                        float scat_pdf = fabsf(wi_z) * (1.0f / kPiF);
+                        float w = power_heuristic(light_pdf, scat_pdf);
+                        c_s = beta * albedo * le * ((1.0f / kPiF) * fabsf(wi_z) * w / light_pdf * nlf);
+                        o_s = offset_origin(p, perr, nrm, pl - p);
+                        float3 tgt = offset_origin(pl, pl_err, nl, o_s - pl);
+                        d_s = tgt - o_s;
+                        tm_s = 1.0f - 0.0001f;
+                        push = true;
                     }
                 }
             }
         }
-        uint32_t s = warp_append(&a.counts[nxt], cont);
-        if (cont) {
-            put_ray(a.rays[nxt], s, o_c, d_c, INFINITY);
-            a.beta[nxt][s] = beta_out;
-            a.rng[nxt][s] = rng_out;
-            a.pid[nxt][s] = id;
-            if (kNrc) a.spread[nxt][s] = spread_next;
-        }
-        uint32_t sl = warp_append(&a.counts[kShadow], push_l);
-        if (push_l) {
-            put_ray(a.srays, sl, o_l, d_l, tm_l);
-            a.scontrib[sl] = make_float4(c_l.x, c_l.y, c_l.z, __uint_as_float(fid));
+        const uint32_t sl = warp_append(&a.counts[kShadow], push);
+        if (push) {
+            put_ray(a.srays, sl, o_s, d_s, tm_s);
+            a.scontrib[sl] = make_float4(c_s.x, c_s.y, c_s.z, __uint_as_float(fid));
             if (kNrc) a.s_train[sl] = make_uint2(tw == kNone ? kNone : tw & kSlotMask, depth);
         }
-        uint32_t sb = warp_append(&a.counts[kShadow], push_b);
-        if (push_b) {
-            put_ray(a.srays, sb, o_b, d_b, tm_b);
-            a.scontrib[sb] = make_float4(c_b.x, c_b.y, c_b.z, __uint_as_float(fid));
+        // the BSDF sample with MIS
+        push = false;
+        if (lk != kNone) {
+            float3 wl = cosine_hemisphere(us0, us1);
+            if (wo_z < 0.0f) wl.z = -wl.z;
+            float3 wb = ss * wl.x + ts * wl.y + nrm * wl.z;
+            float scat_pdf = fabsf(wl.z) * (1.0f / kPiF);
+            float wb_z = dot3(wb, nrm);
+            if (scat_pdf > 0.0f && wb_z * wo_z > 0.0f) {
+                float3 o = offset_origin(p, perr, nrm, wb);
+                TriRay tr = make_tri_ray(o.x, o.y, o.z, wb.x, wb.y, wb.z);
+                const uint32_t lp_id = a.lights[lk];
+                float3 q0 = f3(a.tri[3 * lp_id]), q1 = f3(a.tri[3 * lp_id + 1]), q2 = f3(a.tri[3 * lp_id + 2]);
+                float tl, lb1, lb2;
+                if (triangle_test(tr, q0, q1, q2, INFINITY, tl, lb1, lb2)) {
+                    float4 lg = a.light_geo[lk];
+                    float3 nl = f3(lg);
+                    float3 pli = q0 * (1.0f - lb1 - lb2) + q1 * lb1 + q2 * lb2;
+                    float3 dv = pli - p;
+                    float lpdf = dot3(dv, dv) / (fabsf(dot3(nl, wb)) * lg.w);
+                    if (isfinite(lpdf) && lpdf > 0.0f && dot3(nl, wb) < 0.0f) {
+                        float3 le = f3(a.mat[2 * __float_as_uint(a.tri[3 * lp_id].w) + 1]);
+                        float w = power_heuristic(scat_pdf, lpdf);
+                        c_s = beta * albedo * le * ((1.0f / kPiF) * fabsf(wb_z) * w / scat_pdf * (float)a.n_lights);
+                        o_s = o;
+                        d_s = wb;
+                        tm_s = tl * (1.0f - 0.0001f);
+                        push = true;
+                    }
+                }
+            }
+        }
+        const uint32_t sb = warp_append(&a.counts[kShadow], push);
+        if (push) {
+            put_ray(a.srays, sb, o_s, d_s, tm_s);
+            a.scontrib[sb] = make_float4(c_s.x, c_s.y, c_s.z, __uint_as_float(fid));
             if (kNrc) a.s_train[sb] = make_uint2(tw == kNone ? kNone : tw & kSlotMask, depth);
         }
-        if (kNrc) {
-            uint32_t sq = warp_append(&a.counts[kQueries], query);
-            if (query && sq < a.q_cap) {
-                float* qi = a.q_in + 12 * (size_t)sq;
-                float in[12] = {q_p.x, q_p.y, q_p.z, q_wo.x, q_wo.y, q_wo.z, q_n.x, q_n.y, q_n.z,
-                                q_alb.x, q_alb.y, q_alb.z};
-#pragma unroll
-                for (int q = 0; q < 12; ++q) qi[q] = in[q];
-                a.q_beta[sq] = make_float4(q_beta.x, q_beta.y, q_beta.z, __uint_as_float(fid));
-                a.q_train[sq] = make_uint2(tw == kNone ? kNone : tw & kSlotMask, depth);
+        // the continuation
+        bool cont = false;
+        float pdf = 0.0f;
+        float3 nb;
+        if (live) {
+            float u0 = rng.uniform_float(), u1 = rng.uniform_float();
+            float urr = rng.uniform_float();
+            float3 wl = cosine_hemisphere(u0, u1);
+            if (wo_z < 0.0f) wl.z = -wl.z;
+            float3 wi = ss * wl.x + ts * wl.y + nrm * wl.z;
+            pdf = fabsf(wl.z) * (1.0f / kPiF);
+            float wi_z = dot3(wi, nrm);
+            if (!black && wo_z != 0.0f && pdf > 0.0f && wi_z * wo_z > 0.0f) {
+                nb = beta * albedo * ((1.0f / kPiF) * fabsf(wi_z) / pdf);
+                bool alive = true;
+                if (depth >= a.rr_depth) {
+                    float q = fmaxf(0.05f, 1.0f - max3c(nb));
+                    if (urr < q) alive = false;
+                    else nb = nb * (1.0f / (1.0f - q));
+                }
+                if (alive && depth + 1 < a.max_depth) {
+                    o_s = offset_origin(p, perr, nrm, wi);
+                    d_s = wi;
+                    cont = true;
+                }
             }
+        }
+        const uint32_t s = warp_append(&a.counts[nxt], cont);
+        if (cont) {
+            put_ray(a.rays[nxt], s, o_s, d_s, INFINITY);
+            a.beta[nxt][s] = make_float4(nb.x, nb.y, nb.z, __uint_as_float(fid));
+            a.rng[nxt][s] = make_uint2((uint32_t)rng.state, (uint32_t)(rng.state >> 32));
+            a.pid[nxt][s] = id;
+            if (kNrc) a.spread[nxt][s] = make_float4(sp.x, sp.y, pdf, __uint_as_float(tw));
         }
     }
 }
@@ -614,7 +637,7 @@ cudaError_t bounce(const PtArgs& a, const DeviceAccel& da, const LaunchParams& l
     cudaError_t e = launch_trace(da, a.rays[cur], cap, const_cast<ilm_hit*>(a.hits), nullptr, err, lp, s,
                                  a.counts + cur);
     if (e != cudaSuccess) return e;
-    k_pt_shade<kNrc><<<blocks, 256, 0, s>>>(a, cur);
+    k_pt_shade<kNrc><<<blocks, kShadeBlock, 0, s>>>(a, cur);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     e = launch_trace(da, a.srays, 2ull * cap, nullptr, const_cast<uint32_t*>(a.socc), err, lp, s,
                      a.counts + kShadow);
