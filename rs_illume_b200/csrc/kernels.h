@@ -33,10 +33,9 @@ struct LaunchParams {
                                // testing its own claims (0)
     int split_tail = 0;        // pooled persistent schedule: once the work counter has run out, idle
                                // lanes take stacked subtrees of their warp's unfinished rays
-    int queue_split = 0;       // persistent queries with a device-side count (path queues): the
-                               // one-thread-per-ray split kernel is launched beside the persistent
-                               // one and answers counts of at most one wave; each kernel returns at
-                               // once when the count is the other's
+    int queue_split = 0;       // persistent queries with a device-side count (path queues): counts of at
+                               // most one wave run one thread per ray with the split tail
+    int counter_ready = 0;     // *counter is zero whenever the trace starts (the caller's kernels reset it)
 };
 
 // Everything a trace kernel reads, passed by value.
@@ -56,10 +55,9 @@ struct TraceArgs {
     float bound[6];
     const uint32_t* kd_index;          // kd-tree leaf runs
     uint32_t split_tail = 0;           // LaunchParams::split_tail
-    uint64_t small_max = 0;            // LaunchParams::queue_split: counts up to this go to the
-                                       // one-thread-per-ray kernel (0: no such split)
+    uint32_t counter_ready = 0;        // LaunchParams::counter_ready
     uint32_t warp_rays = 32;           // k_trace_wide_split: rays a warp starts with, a power of two up to
-                                       // 32 (0: from the device-side count)
+                                       // 32
 };
 
 // occ == nullptr: closest hit into `hits`; otherwise any-hit into `occ`.

@@ -55,7 +55,8 @@ namespace {
 // counts[] layout
 enum : int { kQ0 = 0, kQ1 = 1, kShadow = 2, kDepth = 3, kTotClosest = 4, kTotShadow = 5, kDropped = 6,
              kQueries = 7, kTrainSlots = 8, kSamples = 9, kTotQueries = 10, kTotSamples = 11, kFrame = 12,
-             kTrainRows = 13,   // samples gathered by the last frame (kept across renders; trained next frame)
+             kDone = 13,        // blocks of k_pt_accum that have finished
+             kTrainRows = 14,   // samples gathered by the last frame (kept across renders; trained next frame)
              kNumCounts = 16 };
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 // A training path's word: slot (bits 0-23) and the vertices it still goes on
@@ -90,6 +91,7 @@ struct PtArgs {
     float4* scontrib;         // contribution rgb, path id (bits)
     const uint32_t* socc;
     unsigned long long* counts;
+    unsigned long long* trace_counter;   // the traces' work counter: zeroed between any two of them
     // radiance-cache mode
     float4* spread[2];        // s, a0, pdf of the last direction, training word (bits)
     float* q_in;              // queries: 12 floats each
@@ -252,6 +254,7 @@ __global__ void k_pt_camera(PtArgs a, unsigned long long p0, uint32_t count) {
         a.counts[kQ1] = 0;
         a.counts[kShadow] = 0;
         a.counts[kDepth] = 0;
+        *a.trace_counter = 0;
     }
     const bool valid = k < count;
     uint32_t frame = 0;
@@ -305,6 +308,7 @@ __global__ void __launch_bounds__(kShadeBlock, 3) k_pt_shade(PtArgs a, int cur) 
     const uint32_t depth = (uint32_t)a.counts[kDepth];
     const int nxt = cur ^ 1;
     const uint32_t stride = gridDim.x * blockDim.x;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.trace_counter = 0;   // for the shadow trace
     // every lane of a warp runs the same number of iterations (warp_append needs the whole warp)
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t i = base + threadIdx.x;
@@ -534,7 +538,7 @@ __global__ void __launch_bounds__(kShadeBlock, 3) k_pt_shade(PtArgs a, int cur) 
 }
 
 template <bool kNrc>
-__global__ void k_pt_accum(PtArgs a) {
+__global__ void k_pt_accum(PtArgs a, int cur) {
     const uint32_t n = (uint32_t)a.counts[kShadow];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (a.socc[i] != 0u) continue;
@@ -554,14 +558,20 @@ __global__ void k_pt_accum(PtArgs a) {
             }
         }
     }
-}
-
-__global__ void k_pt_advance(PtArgs a, int cur) {
-    a.counts[kTotClosest] += a.counts[cur];
-    a.counts[kTotShadow] += a.counts[kShadow];
-    a.counts[cur] = 0;
-    a.counts[kShadow] = 0;
-    a.counts[kDepth] += 1;
+    // The block that finishes last turns the queues over for the next bounce.
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&a.counts[kDone], 1ull) == gridDim.x - 1) {
+            a.counts[kDone] = 0;
+            a.counts[kTotClosest] += a.counts[cur];
+            a.counts[kTotShadow] += n;
+            a.counts[cur] = 0;
+            a.counts[kShadow] = 0;
+            a.counts[kDepth] += 1;
+            *a.trace_counter = 0;
+        }
+    }
 }
 
 // Flattens the recorded training vertices (at most sample_cap = n_batches *
@@ -630,7 +640,7 @@ __global__ void k_pt_resolve(const float* film, const float* wsum, float* out, u
     }
 }
 
-// One bounce: extend, shade, shadow, accumulate, advance (queue parity cur).
+// One bounce: extend, shade, shadow, accumulate and turn over (queue parity cur).
 template <bool kNrc>
 cudaError_t bounce(const PtArgs& a, const DeviceAccel& da, const LaunchParams& lp, uint32_t cap, uint32_t* err,
                    int cur, int blocks, cudaStream_t s) {
@@ -642,9 +652,7 @@ cudaError_t bounce(const PtArgs& a, const DeviceAccel& da, const LaunchParams& l
     e = launch_trace(da, a.srays, 2ull * cap, nullptr, const_cast<uint32_t*>(a.socc), err, lp, s,
                      a.counts + kShadow);
     if (e != cudaSuccess) return e;
-    k_pt_accum<kNrc><<<blocks, 256, 0, s>>>(a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_pt_advance<<<1, 1, 0, s>>>(a, cur);
+    k_pt_accum<kNrc><<<blocks / 4, 256, 0, s>>>(a, cur);
     return cudaGetLastError();
 }
 
@@ -740,6 +748,8 @@ int32_t setup_render(ilm_context* ctx, PtScene& sc, uint32_t spp, uint32_t max_d
     // thread per ray with the split tail instead.
     r.lp.split_tail = split_tail_of(ctx);
     r.lp.queue_split = r.lp.split_tail;
+    r.lp.counter_ready = 1;
+    a.trace_counter = counter;
     r.err = static_cast<uint32_t*>(ctx->err_word.ptr);
     int dev_sms = 148;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device);

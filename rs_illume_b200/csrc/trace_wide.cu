@@ -56,22 +56,17 @@ __host__ __device__ __forceinline__ uint32_t rays_per_warp(uint64_t n, uint64_t 
 // missed the scene's root box or has finished takes subtrees of its warp's
 // unfinished rays (share_subtrees).  A one-wave query is all tail: its
 // launch lasts as long as its longest rays.
+// Lane `lane` < warp_rays of warp w starts on ray w * warp_rays + lane; the
+// other lanes start idle and help from the first pass.
 template <int W, int kStack, bool kAny, bool kAnalytic>
-__global__ void __launch_bounds__(128) k_trace_wide_split(TraceArgs a) {
+__device__ __forceinline__ void trace_split(const TraceArgs& a, const uint64_t n, const uint32_t warp_rays,
+                                            uint32_t* warp_words) {
     const unsigned lane = threadIdx.x & 31u;
-    // Lane `lane` < warp_rays of warp w starts on ray w * warp_rays + lane;
-    // the other lanes start idle and help from the first pass.
-    __shared__ __align__(16) uint32_t s_warp[4][kWarpWords];
-    uint32_t* warp_words = s_warp[threadIdx.x >> 5];
     uint32_t* ids = warp_words + kPoolWords;
     using Tracer = WideTracer<W, kStack, kAny, kAnalytic>;
     typename Tracer::Entry stk[Tracer::kDepth];
     Tracer T(stk);
     uint32_t st = kFree | (lane << 2);
-    const uint64_t n = ray_count(a);
-    if (a.small_max && n > a.small_max) return;   // the persistent launch beside this one has it
-    const uint32_t warp_rays = a.warp_rays ? a.warp_rays
-                                           : rays_per_warp(n, (uint64_t)gridDim.x * blockDim.x);
     const uint64_t warp_id = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t i = warp_id * warp_rays + lane;
     if (lane < warp_rays && i < n) {
@@ -105,22 +100,21 @@ __global__ void __launch_bounds__(128) k_trace_wide_split(TraceArgs a) {
     }
 }
 
-// kMinBlocks > 0 asks the compiler for that many resident 128-thread blocks
-// per SM (launch_refill).
-// kPool selects how claimed rays reach idle lanes:
-//  * true: the whole warp tests each claimed chunk against the root box, two
-//    rays per lane, answers the misses at full width, and keeps the rays that
-//    enter in a per-warp pool in shared memory; idle lanes take rays from the
-//    pool.  For incoherent batches most rays miss the scene, and this keeps
-//    the lanes that are still traversing from waiting while a few idle lanes
-//    test misses one at a time (5,330 against 4,420 Mrays/s on the 2M-ray
-//    ball workload).  This kernel carries the split tail.
-//  * false: each idle lane tests its own claims, repeating until one enters
-//    (ILM_FLAG_LANE_REFILL); no split tail.
-template <int W, int kStack, bool kAny, int kMinBlocks, bool kAnalytic, bool kPool>
-__global__ void __launch_bounds__(128, kMinBlocks) k_trace_wide_persistent(TraceArgs a) {
-    const uint64_t n = ray_count(a);
-    if (n <= a.small_max) return;                  // the one-thread-per-ray launch beside this one has it
+template <int W, int kStack, bool kAny, bool kAnalytic>
+__global__ void __launch_bounds__(128) k_trace_wide_split(TraceArgs a) {
+    __shared__ __align__(16) uint32_t s_warp[4][kWarpWords];
+    trace_split<W, kStack, kAny, kAnalytic>(a, ray_count(a), a.warp_rays, s_warp[threadIdx.x >> 5]);
+}
+
+// Persistent schedule, pooled refill: the whole warp tests each claimed chunk
+// against the root box, two rays per lane, answers the misses at full width,
+// and keeps the rays that enter in a per-warp pool in shared memory; idle
+// lanes take rays from the pool.  For incoherent batches most rays miss the
+// scene, and this keeps the lanes that are still traversing from waiting
+// while a few idle lanes test misses one at a time (5,330 against 4,420
+// Mrays/s on the 2M-ray ball workload).  It carries the split tail.
+template <int W, int kStack, bool kAny, bool kAnalytic>
+__device__ __forceinline__ void trace_pooled(const TraceArgs& a, const uint64_t n, uint32_t* warp_words) {
     // A short queue (fewer than two rays per resident lane) is claimed one ray
     // per lane, so that its rays run side by side rather than two per lane.
     const unsigned chunk = n < 2ull * gridDim.x * blockDim.x ? 32u : kChunk;
@@ -130,125 +124,162 @@ __global__ void __launch_bounds__(128, kMinBlocks) k_trace_wide_persistent(Trace
     typename Tracer::Entry stk[Tracer::kDepth];
     Tracer T(stk);
     bool exhausted = false;                             // warp-uniform
-    if constexpr (kPool) {
-        __shared__ __align__(16) uint32_t s_warp[4][kWarpWords];
-        uint32_t* warp_words = s_warp[threadIdx.x >> 5];
-        uint32_t* pool = warp_words;                    // offsets of the pooled rays in their chunk
-        uint32_t* ids = warp_words + kPoolWords;        // each lane's ray id (owners)
-        unsigned pool_n = 0;                            // warp-uniform
-        unsigned long long pool_base = 0;               // warp-uniform: the pooled rays' chunk
-        uint32_t st = kFree | (lane << 2);
-        for (;;) {
-            if (!exhausted) {
-                unsigned need = __ballot_sync(0xFFFFFFFFu, role_of(st) == kFree);
-                // Every pass either hands out pooled rays or claims and filters
-                // a chunk (claims are only made with an empty pool), so the
-                // loop ends.
-                while (need != 0u) {
-                    if (pool_n == 0) {
-                        unsigned long long b = 0;
-                        if (lane == 0) b = atomicAdd(a.counter, (unsigned long long)chunk);
-                        b = __shfl_sync(0xFFFFFFFFu, b, 0);
-                        if (b >= n) { exhausted = true; break; }
-                        for (unsigned k = 0; k < chunk; k += 32u) {
-                            const uint64_t rid = b + k + lane;
-                            bool enter = false;
-                            if (rid < n) {
-                                const RayIn r = load_ray(a.rays, rid);
-                                enter = a.n_nodes != 0 && root_enters(r, a.bound);
-                                if (!enter) write_miss(rid, r, a.hits, a.occ);
-                            }
-                            const unsigned m = __ballot_sync(0xFFFFFFFFu, enter);
-                            if (enter) pool[pool_n + __popc(m & below)] = k + lane;
-                            pool_n += __popc(m);
-                        }
-                        __syncwarp();
-                        pool_base = b;
-                        continue;
-                    }
-                    const unsigned rank = __popc(need & below);
-                    const unsigned take = min((unsigned)__popc(need), pool_n);
-                    if (((need >> lane) & 1u) && rank < take) {
-                        const uint64_t id = pool_base + pool[pool_n - 1u - rank];
-                        ids[2 * lane] = (uint32_t)id;
-                        ids[2 * lane + 1] = (uint32_t)(id >> 32);
-                        T.init(load_ray(a.rays, id));
-                        st = kOwner | (lane << 2);
-                    }
-                    pool_n -= take;
-                    __syncwarp();
-                    need = __ballot_sync(0xFFFFFFFFu, role_of(st) == kFree);
-                }
-            }
-            // Subtrees are shared once the counter has run out (warp-uniform).
-            // Before that every busy lane is an owner, and the closest-hit
-            // kernel skips the helpers' bookkeeping (measured 1 % faster); the
-            // any-hit kernel keeps it throughout (2 % faster that way).
-            const bool split_now = exhausted && a.split_tail;
-            const bool tail = kAny || split_now;
-            // A helper of an occluded any-hit ray has nothing left to find.
-            bool owner_occluded = kAny && __shfl_sync(0xFFFFFFFFu, (int)T.occluded, owner_of(st));
-            if (split_now) {
-                share_subtrees<Tracer, kAny>(T, st, owner_occluded, warp_words);
-                // Lanes that just took a subtree have a new owner.
-                if (kAny) owner_occluded = __shfl_sync(0xFFFFFFFFu, (int)T.occluded, owner_of(st));
-            }
-            if (!__any_sync(0xFFFFFFFFu, role_of(st) != kFree)) break;   // only once exhausted
-            const uint32_t role = role_of(st);
-            bool done = false;
-            // An any-hit ray one of its helpers found occluded is finished.
-            if ((role == kOwner || role == kHelper) && owner_occluded) done = true;
-            else if (role == kOwner || role == kHelper) done = T.step(a);
-            if (tail) {
-                const unsigned fin = __ballot_sync(0xFFFFFFFFu, role == kHelper && done);
-                if (fin) merge_helpers<Tracer, kAny>(T, st, fin);
-                if (role == kHelper && done) st = kFree | (lane << 2);
-                if (role == kOwner && done) st = (st & ~3u) | kWaiting;
-                if (role_of(st) == kWaiting && (st >> 8) == 0u) {
-                    T.write((uint64_t)ids[2 * lane] | ((uint64_t)ids[2 * lane + 1] << 32), a);
-                    st = kFree | (lane << 2);
-                }
-            } else if (done) {
-                T.write((uint64_t)ids[2 * lane] | ((uint64_t)ids[2 * lane + 1] << 32), a);
-                st = kFree | (lane << 2);
-            }
-        }
-    } else {
-        bool active = false;
-        uint64_t id = 0;
-        unsigned long long chunk_next = 0, chunk_end = 0;   // warp-uniform
-        for (;;) {
-            unsigned need = __ballot_sync(0xFFFFFFFFu, !active);
-            // Hand rays to idle lanes; rays missing the root box are answered here.
-            // Every pass hands out >= 1 ray or claims a chunk, so the loop ends.
-            while (need != 0u && !exhausted) {
-                if (chunk_next == chunk_end) {
+    uint32_t* pool = warp_words;                    // offsets of the pooled rays in their chunk
+    uint32_t* ids = warp_words + kPoolWords;        // each lane's ray id (owners)
+    unsigned pool_n = 0;                            // warp-uniform
+    unsigned long long pool_base = 0;               // warp-uniform: the pooled rays' chunk
+    uint32_t st = kFree | (lane << 2);
+    for (;;) {
+        if (!exhausted) {
+            unsigned need = __ballot_sync(0xFFFFFFFFu, role_of(st) == kFree);
+            // Every pass either hands out pooled rays or claims and filters
+            // a chunk (claims are only made with an empty pool), so the
+            // loop ends.
+            while (need != 0u) {
+                if (pool_n == 0) {
                     unsigned long long b = 0;
                     if (lane == 0) b = atomicAdd(a.counter, (unsigned long long)chunk);
                     b = __shfl_sync(0xFFFFFFFFu, b, 0);
                     if (b >= n) { exhausted = true; break; }
-                    chunk_next = b;
-                    chunk_end = b + chunk < n ? b + chunk : n;
+                    for (unsigned k = 0; k < chunk; k += 32u) {
+                        const uint64_t rid = b + k + lane;
+                        bool enter = false;
+                        if (rid < n) {
+                            const RayIn r = load_ray(a.rays, rid);
+                            enter = a.n_nodes != 0 && root_enters(r, a.bound);
+                            if (!enter) write_miss(rid, r, a.hits, a.occ);
+                        }
+                        const unsigned m = __ballot_sync(0xFFFFFFFFu, enter);
+                        if (enter) pool[pool_n + __popc(m & below)] = k + lane;
+                        pool_n += __popc(m);
+                    }
+                    __syncwarp();
+                    pool_base = b;
+                    continue;
                 }
-                unsigned avail = (unsigned)(chunk_end - chunk_next);
-                unsigned rank = __popc(need & below);
-                if (((need >> lane) & 1u) && rank < avail) {
-                    id = chunk_next + rank;
-                    RayIn r = load_ray(a.rays, id);
-                    T.init(r);
-                    if (a.n_nodes != 0 && T.enters(a.bound)) active = true;
-                    else write_miss(id, r, a.hits, a.occ);
+                const unsigned rank = __popc(need & below);
+                const unsigned take = min((unsigned)__popc(need), pool_n);
+                if (((need >> lane) & 1u) && rank < take) {
+                    const uint64_t id = pool_base + pool[pool_n - 1u - rank];
+                    ids[2 * lane] = (uint32_t)id;
+                    ids[2 * lane + 1] = (uint32_t)(id >> 32);
+                    T.init(load_ray(a.rays, id));
+                    st = kOwner | (lane << 2);
                 }
-                chunk_next += min((unsigned)__popc(need), avail);
-                need = __ballot_sync(0xFFFFFFFFu, !active);
-            }
-            if (!__any_sync(0xFFFFFFFFu, active)) break;   // only reached once exhausted
-            if (active && T.step(a)) {
-                T.write(id, a);
-                active = false;
+                pool_n -= take;
+                __syncwarp();
+                need = __ballot_sync(0xFFFFFFFFu, role_of(st) == kFree);
             }
         }
+        // Subtrees are shared once the counter has run out (warp-uniform).
+        // Before that every busy lane is an owner, and the closest-hit
+        // kernel skips the helpers' bookkeeping (measured 1 % faster); the
+        // any-hit kernel keeps it throughout (2 % faster that way).
+        const bool split_now = exhausted && a.split_tail;
+        const bool tail = kAny || split_now;
+        // A helper of an occluded any-hit ray has nothing left to find.
+        bool owner_occluded = kAny && __shfl_sync(0xFFFFFFFFu, (int)T.occluded, owner_of(st));
+        if (split_now) {
+            share_subtrees<Tracer, kAny>(T, st, owner_occluded, warp_words);
+            // Lanes that just took a subtree have a new owner.
+            if (kAny) owner_occluded = __shfl_sync(0xFFFFFFFFu, (int)T.occluded, owner_of(st));
+        }
+        if (!__any_sync(0xFFFFFFFFu, role_of(st) != kFree)) break;   // only once exhausted
+        const uint32_t role = role_of(st);
+        bool done = false;
+        // An any-hit ray one of its helpers found occluded is finished.
+        if ((role == kOwner || role == kHelper) && owner_occluded) done = true;
+        else if (role == kOwner || role == kHelper) done = T.step(a);
+        if (tail) {
+            const unsigned fin = __ballot_sync(0xFFFFFFFFu, role == kHelper && done);
+            if (fin) merge_helpers<Tracer, kAny>(T, st, fin);
+            if (role == kHelper && done) st = kFree | (lane << 2);
+            if (role == kOwner && done) st = (st & ~3u) | kWaiting;
+            if (role_of(st) == kWaiting && (st >> 8) == 0u) {
+                T.write((uint64_t)ids[2 * lane] | ((uint64_t)ids[2 * lane + 1] << 32), a);
+                st = kFree | (lane << 2);
+            }
+        } else if (done) {
+            T.write((uint64_t)ids[2 * lane] | ((uint64_t)ids[2 * lane + 1] << 32), a);
+            st = kFree | (lane << 2);
+        }
     }
+}
+
+// Persistent schedule, lane refill: each idle lane tests its own claims,
+// repeating until one enters (ILM_FLAG_LANE_REFILL); no split tail.
+template <int W, int kStack, bool kAny, bool kAnalytic>
+__device__ __forceinline__ void trace_lanes(const TraceArgs& a, const uint64_t n) {
+    // A short queue (fewer than two rays per resident lane) is claimed one ray
+    // per lane, so that its rays run side by side rather than two per lane.
+    const unsigned chunk = n < 2ull * gridDim.x * blockDim.x ? 32u : kChunk;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned below = (1u << lane) - 1u;
+    using Tracer = WideTracer<W, kStack, kAny, kAnalytic>;
+    typename Tracer::Entry stk[Tracer::kDepth];
+    Tracer T(stk);
+    bool exhausted = false;                             // warp-uniform
+    bool active = false;
+    uint64_t id = 0;
+    unsigned long long chunk_next = 0, chunk_end = 0;   // warp-uniform
+    for (;;) {
+        unsigned need = __ballot_sync(0xFFFFFFFFu, !active);
+        // Hand rays to idle lanes; rays missing the root box are answered here.
+        // Every pass hands out >= 1 ray or claims a chunk, so the loop ends.
+        while (need != 0u && !exhausted) {
+            if (chunk_next == chunk_end) {
+                unsigned long long b = 0;
+                if (lane == 0) b = atomicAdd(a.counter, (unsigned long long)chunk);
+                b = __shfl_sync(0xFFFFFFFFu, b, 0);
+                if (b >= n) { exhausted = true; break; }
+                chunk_next = b;
+                chunk_end = b + chunk < n ? b + chunk : n;
+            }
+            unsigned avail = (unsigned)(chunk_end - chunk_next);
+            unsigned rank = __popc(need & below);
+            if (((need >> lane) & 1u) && rank < avail) {
+                id = chunk_next + rank;
+                RayIn r = load_ray(a.rays, id);
+                T.init(r);
+                if (a.n_nodes != 0 && T.enters(a.bound)) active = true;
+                else write_miss(id, r, a.hits, a.occ);
+            }
+            chunk_next += min((unsigned)__popc(need), avail);
+            need = __ballot_sync(0xFFFFFFFFu, !active);
+        }
+        if (!__any_sync(0xFFFFFFFFu, active)) break;   // only reached once exhausted
+        if (active && T.step(a)) {
+            T.write(id, a);
+            active = false;
+        }
+    }
+}
+
+// kMinBlocks > 0 asks the compiler for that many resident 128-thread blocks
+// per SM (launch_refill).
+template <int W, int kStack, bool kAny, int kMinBlocks, bool kAnalytic, bool kPool>
+__global__ void __launch_bounds__(128, kMinBlocks) k_trace_wide_persistent(TraceArgs a) {
+    if constexpr (kPool) {
+        __shared__ __align__(16) uint32_t s_warp[4][kWarpWords];
+        trace_pooled<W, kStack, kAny, kAnalytic>(a, ray_count(a), s_warp[threadIdx.x >> 5]);
+    } else {
+        trace_lanes<W, kStack, kAny, kAnalytic>(a, ray_count(a));
+    }
+}
+
+// A path queue, whose count is known on the device only: at most one ray per
+// thread of the launch runs with the split tail from the start (all of its
+// rays resident at once), a larger count on the pooled schedule.  As two
+// launches, one of which returned at once, and a memset of the work counter
+// before each persistent one, a bounce was nine launches of which five did
+// next to nothing.
+template <int W, int kStack, bool kAny>
+__global__ void __launch_bounds__(128, 7) k_trace_wide_queue(TraceArgs a) {
+    __shared__ __align__(16) uint32_t s_warp[4][kWarpWords];
+    uint32_t* warp_words = s_warp[threadIdx.x >> 5];
+    const uint64_t n = ray_count(a), threads = (uint64_t)gridDim.x * blockDim.x;
+    if (n <= threads) trace_split<W, kStack, kAny, false>(a, n, rays_per_warp(n, threads), warp_words);
+    else trace_pooled<W, kStack, kAny, false>(a, n, warp_words);
 }
 
 template <int W, int kStack, int kMinBlocks, bool kAnalytic, bool kPool>
@@ -260,8 +291,10 @@ cudaError_t launch_persistent(const TraceArgs& t, cudaStream_t s) {
     if (grid == 0) return cudaErrorInvalidConfiguration;
     const uint64_t need_blocks = (t.n + block - 1) / block;
     if (grid > need_blocks) grid = need_blocks;
-    cudaError_t e = cudaMemsetAsync(t.counter, 0, sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
+    if (!t.counter_ready) {
+        cudaError_t e = cudaMemsetAsync(t.counter, 0, sizeof(unsigned long long), s);
+        if (e != cudaSuccess) return e;
+    }
     if (t.occ) ka<<<(unsigned)grid, block, 0, s>>>(t);
     else kc<<<(unsigned)grid, block, 0, s>>>(t);
     return cudaGetLastError();
@@ -289,25 +322,22 @@ template <int W, int kStack, bool kAnalytic>
 cudaError_t launch_variant(const TraceArgs& t, const LaunchParams& lp, cudaStream_t s) {
     const unsigned block = 128;
     if (lp.persistent && t.counter) {
-        if (lp.queue_split && t.n_dev && t.split_tail) {
-            // A queue whose count is known on the device only: a count of at
-            // most one wave of the split kernel runs there (all of its rays
-            // resident at once, idle lanes helping from the start), a larger
-            // one on the persistent kernel.  The launch has a warp for every
-            // ray that the queue can hold, up to one wave.
-            auto kc = k_trace_wide_split<W, kStack, false, kAnalytic>;
-            auto ka = k_trace_wide_split<W, kStack, true, kAnalytic>;
-            const uint64_t wave_blocks = resident_blocks(t.occ ? (const void*)ka : (const void*)kc, (int)block);
-            const uint64_t blocks = std::min<uint64_t>(wave_blocks, (t.n + block / 32 - 1) / (block / 32));
-            if (blocks > 0) {
-                TraceArgs q = t;
-                q.small_max = blocks * block;
-                q.warp_rays = 0;                    // from the device-side count (rays_per_warp)
-                if (t.occ) ka<<<(unsigned)blocks, block, 0, s>>>(q);
-                else kc<<<(unsigned)blocks, block, 0, s>>>(q);
-                cudaError_t e = cudaGetLastError();
-                if (e != cudaSuccess) return e;
-                return launch_refill<W, kStack, kAnalytic>(q, lp, s);
+        if constexpr (!kAnalytic) {
+            if (lp.queue_split && t.n_dev && t.split_tail) {
+                auto kc = k_trace_wide_queue<W, kStack, false>;
+                auto ka = k_trace_wide_queue<W, kStack, true>;
+                // a warp for every ray that the queue can hold, up to one wave
+                const uint64_t grid =
+                    std::min<uint64_t>(resident_blocks(t.occ ? (const void*)ka : (const void*)kc, (int)block),
+                                       (t.n + block / 32 - 1) / (block / 32));
+                if (grid == 0) return cudaErrorInvalidConfiguration;
+                if (!t.counter_ready) {
+                    cudaError_t e = cudaMemsetAsync(t.counter, 0, sizeof(unsigned long long), s);
+                    if (e != cudaSuccess) return e;
+                }
+                if (t.occ) ka<<<(unsigned)grid, block, 0, s>>>(t);
+                else kc<<<(unsigned)grid, block, 0, s>>>(t);
+                return cudaGetLastError();
             }
         }
         return launch_refill<W, kStack, kAnalytic>(t, lp, s);
