@@ -422,7 +422,7 @@ typedef struct {
     uint32_t rr_depth;     /* Russian roulette from this bounce on (3) */
     uint64_t seed;
     uint32_t wave_paths;   /* paths in flight per wave (0 = 2^21) */
-    int32_t use_graphs;    /* replay each bounce as a CUDA graph */
+    int32_t use_graphs;    /* replay each bounce as a CUDA graph (in renders of four waves or more) */
     ilm_filter_desc filter; /* film filter (FilmTile::add_sample, film.rs:288-333); radius 0 or the box
                                of radius 0.5: each sample counts in its own pixel */
 } ilm_pt_opts;
@@ -492,7 +492,7 @@ int32_t ilm_nrc_encode(ilm_context* ctx, ilm_nrc* nrc, const float* inputs, uint
  * paths per frame) runs to the end and its vertices become training samples
  * (at most train_samples per frame); after each frame (if `train`) the network
  * takes train_steps Adam steps on interleaved subsets of them.  A frame runs on
- * the device as one CUDA graph; with a time budget, frames are launched until
+ * the device as one CUDA graph (from four frames on); with a time budget, frames are launched until
  * the finished ones reach it (the frame queued by then is completed and
  * counted). */
 typedef struct {

@@ -21,7 +21,8 @@
 //   accum   unoccluded contributions -> film (float atomics)
 // Queues are compacted with a warp ballot, a prefix popcount and one atomicAdd
 // per warp.  Queue sizes live in device memory, so a bounce is a fixed launch
-// sequence, captured once per queue parity as a CUDA graph and replayed.
+// sequence, captured once per queue parity as a CUDA graph and replayed in
+// renders of several waves.
 //
 // Radiance-cache mode (kNrc): each path tracks its spread
 //   a0 = d1^2 / (4 pi |cos1|),  s_n = sum_{i=2..n} sqrt(d_i^2 / (pdf_{i-1} |cos_i|)),
@@ -900,7 +901,12 @@ int32_t ilm_render_pt(ilm_context* ctx, ilm_pt_scene_id scene, const ilm_pt_opts
     cudaStream_t s = r.s;
     cudaError_t e = cudaSuccess;
     cudaGraphExec_t graphs[2] = {nullptr, nullptr};
-    if (opts->use_graphs) {
+    // Capturing and instantiating the two bounces costs 100 to 120 us and a
+    // replay saves 25 us a wave: below four waves the bounces are launched one
+    // by one (64 x 64 at 1 spp 536 against 657 us, 1024 x 1024 at 4 spp, two
+    // waves, 8,762 against 8,831; at 16 spp, eight waves, 34,936 against 34,742).
+    const bool use_graphs = opts->use_graphs && (r.total + r.P - 1) / r.P >= 4;
+    if (use_graphs) {
         // One eager bounce over empty queues (every kernel returns at once)
         // does the launchers' one-time setup outside the capture.
         if ((e = bounce<false>(a, r.da, r.lp, r.P, r.err, 0, r.blocks, s)) != cudaSuccess)
@@ -925,7 +931,7 @@ int32_t ilm_render_pt(ilm_context* ctx, ilm_pt_scene_id scene, const ilm_pt_opts
         k_pt_camera<false><<<(cnt + 255) / 256, 256, 0, s>>>(a, p0, cnt);
         for (uint32_t depth = 0; depth < opts->max_depth; ++depth) {
             int cur = depth & 1;
-            if (opts->use_graphs) e = cudaGraphLaunch(graphs[cur], s);
+            if (use_graphs) e = cudaGraphLaunch(graphs[cur], s);
             else e = bounce<false>(a, r.da, r.lp, r.P, r.err, cur, r.blocks, s);
             if (e != cudaSuccess) break;
         }
@@ -1063,11 +1069,16 @@ int32_t ilm_render_nrc(ilm_context* ctx, ilm_pt_scene_id scene, ilm_nrc* nrc, co
         k_nrc_tally<<<1, 1, 0, s>>>(a, sample_cap);
         return cudaGetLastError();
     };
-    // one eager bounce over the empty queues does the launchers' one-time
-    // setup outside the capture
-    if ((e = bounce<true>(a, r.da, r.lp, P, r.err, 0, r.blocks, s)) != cudaSuccess) return cuda_fail(ctx, e, "bounce");
+    // Capture and instantiation cost 150 us and a replay saves 45 us a frame:
+    // below four frames each is enqueued as it is (128 x 128, one frame 560
+    // against 726 us, four 1,818 against 1,806, sixteen 6,643 against 5,848).
+    const bool use_graph = max_frames >= 4;
     cudaGraphExec_t frame_graph = nullptr;
-    {
+    if (use_graph) {
+        // one eager bounce over the empty queues does the launchers' one-time
+        // setup outside the capture
+        if ((e = bounce<true>(a, r.da, r.lp, P, r.err, 0, r.blocks, s)) != cudaSuccess)
+            return cuda_fail(ctx, e, "bounce");
         cudaGraph_t g = nullptr;
         if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
             return cuda_fail(ctx, e, "cudaStreamBeginCapture");
@@ -1086,7 +1097,7 @@ int32_t ilm_render_nrc(ilm_context* ctx, ilm_pt_scene_id scene, ilm_nrc* nrc, co
     cudaEventRecord(b.ev0, s);
     uint32_t frame = 0;
     for (; frame < max_frames; ++frame) {
-        if ((e = cudaGraphLaunch(frame_graph, s)) != cudaSuccess) break;
+        if ((e = use_graph ? cudaGraphLaunch(frame_graph, s) : enqueue_frame()) != cudaSuccess) break;
         cudaEventRecord(done[frame & 1], s);
         if (o->time_budget_s > 0.0 && frame >= 1) {
             if ((e = cudaEventSynchronize(done[(frame - 1) & 1])) != cudaSuccess) break;
@@ -1096,7 +1107,7 @@ int32_t ilm_render_nrc(ilm_context* ctx, ilm_pt_scene_id scene, ilm_nrc* nrc, co
         }
     }
     cudaEventRecord(b.ev1, s);
-    cudaGraphExecDestroy(frame_graph);
+    if (frame_graph) cudaGraphExecDestroy(frame_graph);
     if (e != cudaSuccess) {
         cudaEventDestroy(done[0]);
         cudaEventDestroy(done[1]);
