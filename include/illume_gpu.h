@@ -165,7 +165,10 @@ const char* ilm_last_error_string(const ilm_context* ctx);
  * staging: copy-in and copy-out run on their own streams (the host link
  * carries both directions at once) and a ring of four slots traces on four
  * streams; the first and last chunks ramp from chunk/8.  4096 .. 2^24,
- * default 524288. */
+ * default 524288.  Once 2^21 rays have come from pageable buffers in queries
+ * of 8192 rays or more, the context keeps 8 MB of pinned memory and up to seven
+ * copying threads (idle between calls) for such queries, whose chunks are then
+ * at most 43690 rays; both go with the context. */
 int32_t ilm_context_set_stage_chunk(ilm_context* ctx, uint64_t rays);
 
 /* One segment of a cubic Bezier curve (shapes/curve.rs:14-91): the curve's

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "builder.h"
+#include "host_copy.h"
 #include "illume_gpu.h"
 #include "kernels.h"
 #include "layout.h"
@@ -112,6 +113,8 @@ struct ilm_context {
     cudaEvent_t fence = nullptr;
     ilm::Stage stage[ilm::kStageSlots];
     uint64_t stage_chunk = 1ull << 19;
+    uint64_t pageable_rays = 0;                  // until `staging` is made
+    std::unique_ptr<ilm::HostStaging> staging;   // see kPageableRent
     ilm::DeviceBuffer err_word;
     std::string last_error;
     std::map<ilm_mesh_id, std::unique_ptr<ilm::Mesh>> meshes;
