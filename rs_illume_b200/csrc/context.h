@@ -48,9 +48,9 @@ struct Mesh {
 // vertices and attributes of all its triangle meshes, concatenated, and per
 // primitive id its three global vertex indices and its mesh slot.
 struct ShadingData {
-    DeviceBuffer vtx, nrm, tan, uv;  // float4, float4, float4, float2 per vertex
-    DeviceBuffer tri;                // uint4 per primitive: i0, i1, i2, mesh slot (kShadeSphere for spheres)
-    DeviceBuffer mesh;               // uint32 flags per mesh slot
+    DeviceBuffer vtx;   // two float4 per vertex: position and u, normal and v
+    DeviceBuffer tan;   // float4 per vertex
+    DeviceBuffer tri;   // uint4 per primitive: i0, i1, i2, mesh flags (kShadeSphere for spheres)
     bool ready = false;
 };
 

@@ -13,7 +13,8 @@
 // as the geometric one, n, dpdu, dpdv, dndu, dndv, as in pbrt).
 #include <cuda_runtime.h>
 
-#include <cstring>
+#include <cstddef>
+#include <memory>
 #include <vector>
 
 #include "context.h"
@@ -59,27 +60,26 @@ __device__ __forceinline__ V3 interp(float b0, float b1, float b2, V3 a, V3 b, V
     return vadd(vadd(vmul(b0, a), vmul(b1, b)), vmul(b2, c));
 }
 
-// Vertex tables: positions, normals and tangents as float4 (w unused), so a
-// vertex is one 16-byte load.
+// A vertex is one 32-byte sector: its position and normal with u and v in the
+// fourth words (zeros where the mesh has none).  A triangle is its vertices and
+// its mesh's flags, or kShadeSphere.
 struct ShadeArgs {
-    const float4* vtx;
-    const float4* nrm;
+    const float4* vtx;   // two per vertex
     const float4* tan;
-    const float2* uv;
     const uint4* tri;
-    const uint32_t* mesh;
     uint32_t n_prims;
 };
 
-__device__ __forceinline__ V3 load3(const float4* a, uint32_t i) {
-    const float4 v = __ldg(a + i);
-    return {v.x, v.y, v.z};
-}
-__device__ __forceinline__ void put3(float* d, V3 v) { d[0] = v.x; d[1] = v.y; d[2] = v.z; }
-
+__device__ __forceinline__ V3 xyz(float4 v) { return {v.x, v.y, v.z}; }
 constexpr int kSiBlock = 128;
 constexpr int kSiWords = sizeof(ilm_surface_interaction) / 4;   // 44
 static_assert(sizeof(ilm_surface_interaction) == 176 && kSiWords % 4 == 0, "records are 11 16-byte words");
+
+static_assert(offsetof(ilm_surface_interaction, n) == 24 && offsetof(ilm_surface_interaction, dpdu) == 44 &&
+                  offsetof(ilm_surface_interaction, shading_n) == 92 &&
+                  offsetof(ilm_surface_interaction, shading_dndu) == 128 &&
+                  offsetof(ilm_surface_interaction, wo) == 152 && offsetof(ilm_surface_interaction, kind) == 172,
+              "the words written below");
 
 // Record i of a 16-byte aligned array, else word by word.
 template <bool kAligned, class T>
@@ -99,37 +99,42 @@ __device__ __forceinline__ T load_record(const T* p, uint64_t i) {
     return v;
 }
 
-// The SurfaceInteraction of one (ray, hit) pair.
+// A record with no more than its primitive, distance, kind, direction and point.
+__device__ __forceinline__ void put_plain(float4* rec, const ilm_hit& h, uint32_t kind, V3 wo, V3 p) {
+    rec[0] = make_float4(p.x, p.y, p.z, 0.0f);
+#pragma unroll
+    for (int k = 1; k < 9; ++k) rec[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    rec[9] = make_float4(0.0f, 0.0f, wo.x, wo.y);
+    rec[10] = make_float4(wo.z, h.t, __uint_as_float(h.prim), __uint_as_float(kind));
+}
+
+// The SurfaceInteraction of one (ray, hit) pair, written to `rec` (11 16-byte
+// words) in pieces as they are known: 44 words held to the end cost the
+// registers of two resident blocks.
 __device__ __forceinline__ void surface_interaction(const ShadeArgs& sa, const ilm_ray& r, const ilm_hit& h,
-                                                    ilm_surface_interaction& si) {
-    memset(&si, 0, sizeof si);
-    si.prim = h.prim;
-    si.t = h.t;
-    si.kind = ILM_SI_MISS;
-    const V3 o{r.o[0], r.o[1], r.o[2]}, d{r.d[0], r.d[1], r.d[2]};
-    if (h.prim >= sa.n_prims) return;   // miss (or a flagged traversal error)
-    put3(si.wo, vneg(d));
-    const uint4 tv = sa.tri[h.prim];
-    if (tv.w == kShadeSphere) {
-        si.kind = ILM_SI_SPHERE;
-        put3(si.p, vadd(o, vmul(h.t, d)));
-        return;
-    }
-    const uint32_t flags = sa.mesh[tv.w];
-    const V3 p0 = load3(sa.vtx, tv.x), p1 = load3(sa.vtx, tv.y), p2 = load3(sa.vtx, tv.z);
+                                                    float4* rec) {
+    const V3 o{r.o[0], r.o[1], r.o[2]}, d{r.d[0], r.d[1], r.d[2]}, zero{0.0f, 0.0f, 0.0f};
+    if (h.prim >= sa.n_prims) return put_plain(rec, h, ILM_SI_MISS, zero, zero);   // or a flagged traversal error
+    const uint4 tv = __ldg(sa.tri + h.prim);
+    if (tv.w == kShadeSphere) return put_plain(rec, h, ILM_SI_SPHERE, vneg(d), vadd(o, vmul(h.t, d)));
+    const uint32_t flags = tv.w;
+    // all that the record may need is asked for at once
+    const float4 *va = sa.vtx + 2ull * tv.x, *vb = sa.vtx + 2ull * tv.y, *vc = sa.vtx + 2ull * tv.z;
+    const float4 pa = __ldg(va), pb = __ldg(vb), pc = __ldg(vc);
+    const float4 na = __ldg(va + 1), nb = __ldg(vb + 1), nc = __ldg(vc + 1);
+    const V3 p0 = xyz(pa), p1 = xyz(pb), p2 = xyz(pc);
     // barycentrics of the hit, as the traversal computed them
     TriRay tr = make_tri_ray(o.x, o.y, o.z, d.x, d.y, d.z);
     float t, b0, b1, b2;
     if (!triangle_test(tr, make_float3(p0.x, p0.y, p0.z), make_float3(p1.x, p1.y, p1.z),
                        make_float3(p2.x, p2.y, p2.z), INFINITY, t, b1, b2, &b0))
-        return;   // not a hit of this triangle: left as a miss
+        return put_plain(rec, h, ILM_SI_MISS, vneg(d), zero);   // not a hit of this triangle
     // uv parameterisation (triangle.rs:96-112; default (0,0), (1,0), (1,1))
     float uv0[2] = {0.0f, 0.0f}, uv1[2] = {1.0f, 0.0f}, uv2[2] = {1.0f, 1.0f};
     if (flags & kHasUV) {
-        const float2 a = __ldg(sa.uv + tv.x), b = __ldg(sa.uv + tv.y), c = __ldg(sa.uv + tv.z);
-        uv0[0] = a.x; uv0[1] = a.y;
-        uv1[0] = b.x; uv1[1] = b.y;
-        uv2[0] = c.x; uv2[1] = c.y;
+        uv0[0] = pa.w; uv0[1] = na.w;
+        uv1[0] = pb.w; uv1[1] = nb.w;
+        uv2[0] = pc.w; uv2[1] = nc.w;
     }
     // partial derivatives (triangle.rs:264-292)
     const float duv02x = __fsub_rn(uv0[0], uv2[0]), duv02y = __fsub_rn(uv0[1], uv2[1]);
@@ -145,7 +150,8 @@ __device__ __forceinline__ void surface_interaction(const ShadeArgs& sa, const i
     }
     if (degenerate_uv || vlen2(vcross(dpdu, dpdv)) == 0.0f) {
         const V3 ng = vcross(vsub(p2, p0), vsub(p1, p0));
-        if (vlen2(ng) == 0.0f) return;   // degenerate triangle: the reference reports no hit
+        if (vlen2(ng) == 0.0f)   // degenerate triangle: the reference reports no hit
+            return put_plain(rec, h, ILM_SI_MISS, vneg(d), zero);
         coordinate_system(vnormalize(ng), dpdu, dpdv);
     }
     // error bound and hit point (triangle.rs:295-305)
@@ -156,8 +162,15 @@ __device__ __forceinline__ void surface_interaction(const ShadeArgs& sa, const i
                   __fmul_rn(kGamma7, __fadd_rn(__fadd_rn(fabsf(__fmul_rn(b0, p0.z)), fabsf(__fmul_rn(b1, p1.z))),
                                              fabsf(__fmul_rn(b2, p2.z))))};
     const V3 phit = interp(b0, b1, b2, p0, p1, p2);
-    si.uv[0] = __fadd_rn(__fadd_rn(__fmul_rn(b0, uv0[0]), __fmul_rn(b1, uv1[0])), __fmul_rn(b2, uv2[0]));
-    si.uv[1] = __fadd_rn(__fadd_rn(__fmul_rn(b0, uv0[1]), __fmul_rn(b1, uv1[1])), __fmul_rn(b2, uv2[1]));
+    rec[0] = make_float4(phit.x, phit.y, phit.z, perr.x);
+    rec[1] = make_float4(perr.y, perr.z, 0.0f, 0.0f);   // n.x, n.y follow
+    rec[2] = make_float4(0.0f, __fadd_rn(__fadd_rn(__fmul_rn(b0, uv0[0]), __fmul_rn(b1, uv1[0])), __fmul_rn(b2, uv2[0])),
+                         __fadd_rn(__fadd_rn(__fmul_rn(b0, uv0[1]), __fmul_rn(b1, uv1[1])), __fmul_rn(b2, uv2[1])),
+                         dpdu.x);                       // n.z follows
+    rec[3] = make_float4(dpdu.y, dpdu.z, dpdv.x, dpdv.y);
+    rec[4] = make_float4(dpdv.z, 0.0f, 0.0f, 0.0f);
+    rec[9] = make_float4(0.0f, 0.0f, -d.x, -d.y);       // shading_dndv.y and .z follow
+    rec[10] = make_float4(-d.z, t, __uint_as_float(h.prim), __uint_as_float((uint32_t)ILM_SI_TRIANGLE));
     const bool reverse = (flags & kReverse) != 0;   // world-space meshes: no handedness swap
     // SurfaceInteraction::new (interaction.rs:262-316) then the triangle's
     // normal override (triangle.rs:322-331)
@@ -168,12 +181,12 @@ __device__ __forceinline__ void surface_interaction(const ShadeArgs& sa, const i
         // shading geometry (triangle.rs:333-414)
         V3 ns = nrm;
         if (flags & kHasN) {
-            V3 nn = interp(b0, b1, b2, load3(sa.nrm, tv.x), load3(sa.nrm, tv.y), load3(sa.nrm, tv.z));
+            V3 nn = interp(b0, b1, b2, xyz(na), xyz(nb), xyz(nc));
             if (vlen2(nn) > 0.0f) ns = vnormalize(nn);
         }
         V3 ss = vnormalize(dpdu);
         if (flags & kHasS) {
-            V3 s = interp(b0, b1, b2, load3(sa.tan, tv.x), load3(sa.tan, tv.y), load3(sa.tan, tv.z));
+            V3 s = interp(b0, b1, b2, xyz(__ldg(sa.tan + tv.x)), xyz(__ldg(sa.tan + tv.y)), xyz(__ldg(sa.tan + tv.z)));
             if (vlen2(s) > 0.0f) ss = vnormalize(s);
         }
         V3 ts = vcross(ss, ns);
@@ -185,7 +198,7 @@ __device__ __forceinline__ void surface_interaction(const ShadeArgs& sa, const i
         }
         V3 dndu{0, 0, 0}, dndv{0, 0, 0};
         if (flags & kHasN) {
-            const V3 n0 = load3(sa.nrm, tv.x), n1 = load3(sa.nrm, tv.y), n2 = load3(sa.nrm, tv.z);
+            const V3 n0 = xyz(na), n1 = xyz(nb), n2 = xyz(nc);
             const V3 dn1 = vsub(n0, n2), dn2 = vsub(n1, n2);
             const float det2 = __fsub_rn(__fmul_rn(duv02x, duv12y), __fmul_rn(duv02y, duv12x));
             if (fabsf(det2) < 1e-8f) {
@@ -203,12 +216,13 @@ __device__ __forceinline__ void surface_interaction(const ShadeArgs& sa, const i
         if (vdot(nrm, sn) < 0.0f) nrm = vneg(nrm);
         sdpdu = ss; sdpdv = ts; sdndu = dndu; sdndv = dndv;
     }
-    si.kind = ILM_SI_TRIANGLE;
-    si.t = t;
-    put3(si.p, phit); put3(si.p_error, perr); put3(si.n, nrm);
-    put3(si.dpdu, dpdu); put3(si.dpdv, dpdv);
-    put3(si.shading_n, sn); put3(si.shading_dpdu, sdpdu); put3(si.shading_dpdv, sdpdv);
-    put3(si.shading_dndu, sdndu); put3(si.shading_dndv, sdndv);
+    reinterpret_cast<float2*>(rec + 1)[1] = make_float2(nrm.x, nrm.y);
+    reinterpret_cast<float*>(rec + 2)[0] = nrm.z;
+    rec[5] = make_float4(0.0f, 0.0f, 0.0f, sn.x);
+    rec[6] = make_float4(sn.y, sn.z, sdpdu.x, sdpdu.y);
+    rec[7] = make_float4(sdpdu.z, sdpdv.x, sdpdv.y, sdpdv.z);
+    rec[8] = make_float4(sdndu.x, sdndu.y, sdndu.z, sdndv.x);
+    reinterpret_cast<float2*>(rec + 9)[0] = make_float2(sdndv.y, sdndv.z);
 }
 
 // One thread per (ray, hit).  The kernel streams 48 bytes in and 176 out per
@@ -218,27 +232,27 @@ __device__ __forceinline__ void surface_interaction(const ShadeArgs& sa, const i
 // Each warp therefore lays its 32 records out in shared memory (16-byte
 // stores at a 176-byte stride: eight consecutive lanes touch eight different
 // bank groups, since 11 is odd) and hands the 5,632 contiguous bytes to one
-// bulk copy: 79 us, 3,430 GB/s.  kAligned: rays, hits and out on 16-byte boundaries (every
+// bulk copy: 79 us.  What was left was the wait on four loads in a chain (hit,
+// triangle, mesh flags and positions, then normals and uvs) with 20 warps an SM
+// to hide it: vertices of one sector each, read at once, 67 us; the words of a
+// record written as they are known, which frees the registers of three more
+// blocks, 53 us (8 blocks; 55 at 7, 68 at 9, which spill), 4,430 GB/s of the 48
+// and 176 bytes.  kAligned: rays, hits and out on 16-byte boundaries (every
 // buffer a query accepts is; this entry point also takes 4-byte aligned ones,
 // which are read and written word by word, the writes still coalesced).
 template <bool kAligned>
-__global__ void __launch_bounds__(kSiBlock) k_surface_interactions(ShadeArgs sa, const ilm_ray* __restrict__ rays,
+__global__ void __launch_bounds__(kSiBlock, 8) k_surface_interactions(ShadeArgs sa, const ilm_ray* __restrict__ rays,
                                                                    const ilm_hit* __restrict__ hits, uint64_t n,
                                                                    ilm_surface_interaction* __restrict__ out) {
-    __shared__ __align__(16) uint4 s_rec[kSiBlock / 32][32 * kSiWords / 4];
+    __shared__ __align__(16) float4 s_rec[kSiBlock / 32][32 * kSiWords / 4];
     const uint32_t lane = threadIdx.x & 31u;
-    uint4* warp_rec = s_rec[threadIdx.x >> 5];
+    float4* warp_rec = s_rec[threadIdx.x >> 5];
     const uint64_t first = (uint64_t)blockIdx.x * kSiBlock + (threadIdx.x & ~31u);   // the warp's first record
     if (first >= n) return;
     const uint32_t rows = n - first < 32u ? (uint32_t)(n - first) : 32u;
-    if (lane < rows) {
-        __align__(16) ilm_surface_interaction si;
+    if (lane < rows)
         surface_interaction(sa, load_record<kAligned>(rays, first + lane), load_record<kAligned>(hits, first + lane),
-                            si);
-#pragma unroll
-        for (int k = 0; k < kSiWords / 4; ++k)
-            warp_rec[lane * (kSiWords / 4) + k] = reinterpret_cast<const uint4*>(&si)[k];
-    }
+                            warp_rec + lane * (kSiWords / 4));
     if constexpr (kAligned) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // this lane's record, visible to the copy
         __syncwarp();
@@ -271,46 +285,48 @@ cudaError_t launch_interactions(const ShadeArgs& sa, const ilm_ray* rays, const 
 int32_t ensure_shading(ilm_context* ctx, Accel& acc) {
     ShadingData& sd = acc.shading;
     if (sd.ready) return ILM_OK;
-    std::vector<float4> vtx, nrm, tan;
-    std::vector<float2> uv;
-    std::vector<uint4> tri;
-    std::vector<uint32_t> mesh;
-    for (size_t k = 0; k < acc.mesh_ids.size(); ++k) {
-        auto it = ctx->meshes.find(acc.mesh_ids[k]);
+    size_t nv = 0, nt = 0;
+    bool tangents = false;
+    for (ilm_mesh_id id : acc.mesh_ids) {
+        auto it = ctx->meshes.find(id);
         if (it == ctx->meshes.end()) { set_error(ctx, "surface interactions: a mesh of the accel is gone"); return ILM_ERR_NOT_FOUND; }
         const Mesh& m = *it->second;
+        if (!m.is_spheres) nv += m.xyz.size() / 3;
+        nt += m.n_prims;
+        tangents = tangents || (!m.is_spheres && !m.s.empty());
+    }
+    // uninitialised: every element that a triangle names is written below
+    std::unique_ptr<float4[]> vtx(new float4[2 * nv + 2]), tan(new float4[tangents ? nv + 1 : 1]);
+    std::unique_ptr<uint4[]> tri(new uint4[nt + 1]);
+    size_t v0 = 0, t0 = 0;
+    for (ilm_mesh_id id : acc.mesh_ids) {
+        const Mesh& m = *ctx->meshes.find(id)->second;
         if (m.is_spheres) {
-            for (uint32_t p = 0; p < m.n_prims; ++p) tri.push_back(make_uint4(0, 0, 0, kShadeSphere));
+            for (uint32_t p = 0; p < m.n_prims; ++p) tri[t0++] = make_uint4(0, 0, 0, kShadeSphere);
             continue;
         }
-        const uint32_t base = (uint32_t)vtx.size(), nv = (uint32_t)(m.xyz.size() / 3);
-        auto append = [&](std::vector<float4>& dst, const std::vector<float>& src) {
-            const size_t at = dst.size();
-            dst.resize(at + nv, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-            if (!src.empty())
-                for (uint32_t k = 0; k < nv; ++k)
-                    dst[at + k] = make_float4(src[3 * k], src[3 * k + 1], src[3 * k + 2], 0.0f);
+        const size_t n = m.xyz.size() / 3;
+        auto at = [](const std::vector<float>& src, size_t v, float w) {
+            return src.empty() ? make_float4(0.0f, 0.0f, 0.0f, w)
+                               : make_float4(src[3 * v], src[3 * v + 1], src[3 * v + 2], w);
         };
-        append(vtx, m.xyz);
-        append(nrm, m.n);
-        append(tan, m.s);
-        uv.resize(uv.size() + nv, make_float2(0.0f, 0.0f));
-        for (uint32_t k = 0; k < nv && !m.uv.empty(); ++k) uv[base + k] = make_float2(m.uv[2 * k], m.uv[2 * k + 1]);
-        uint32_t flags = (m.n.empty() ? 0u : (uint32_t)kHasN) | (m.s.empty() ? 0u : (uint32_t)kHasS) |
-                         (m.uv.empty() ? 0u : (uint32_t)kHasUV) | (m.reverse ? (uint32_t)kReverse : 0u);
-        const uint32_t slot = (uint32_t)mesh.size();
-        mesh.push_back(flags);
+        for (size_t v = 0; v < n; ++v) {
+            vtx[2 * (v0 + v)] = at(m.xyz, v, m.uv.empty() ? 0.0f : m.uv[2 * v]);
+            vtx[2 * (v0 + v) + 1] = at(m.n, v, m.uv.empty() ? 0.0f : m.uv[2 * v + 1]);
+        }
+        for (size_t v = 0; v < n && tangents; ++v) tan[v0 + v] = at(m.s, v, 0.0f);
+        const uint32_t flags = (m.n.empty() ? 0u : (uint32_t)kHasN) | (m.s.empty() ? 0u : (uint32_t)kHasS) |
+                               (m.uv.empty() ? 0u : (uint32_t)kHasUV) | (m.reverse ? (uint32_t)kReverse : 0u);
+        const uint32_t base = (uint32_t)v0;
         for (uint32_t p = 0; p < m.n_prims; ++p)
-            tri.push_back(make_uint4(base + m.idx[3 * p], base + m.idx[3 * p + 1], base + m.idx[3 * p + 2], slot));
+            tri[t0++] = make_uint4(base + m.idx[3 * p], base + m.idx[3 * p + 1], base + m.idx[3 * p + 2], flags);
+        v0 += n;
     }
-    if (mesh.empty()) mesh.push_back(0);
-    if (vtx.empty()) { vtx.resize(1); nrm.resize(1); tan.resize(1); uv.resize(1); }
-    if (tri.empty()) tri.push_back(make_uint4(0, 0, 0, kShadeSphere));
     cudaError_t e;
     struct Up { DeviceBuffer& b; const void* src; size_t bytes; } ups[] = {
-        {sd.vtx, vtx.data(), vtx.size() * 16}, {sd.nrm, nrm.data(), nrm.size() * 16}, {sd.tan, tan.data(), tan.size() * 16},
-        {sd.uv, uv.data(), uv.size() * 8},     {sd.tri, tri.data(), tri.size() * 16}, {sd.mesh, mesh.data(), mesh.size() * 4}};
+        {sd.vtx, vtx.get(), nv * 32}, {sd.tan, tan.get(), tangents ? nv * 16 : 0}, {sd.tri, tri.get(), nt * 16}};
     for (auto& u : ups) {
+        if (u.bytes == 0) continue;
         if ((e = u.b.reserve(u.bytes)) != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(shading)");
         if ((e = cudaMemcpy(u.b.ptr, u.src, u.bytes, cudaMemcpyHostToDevice)) != cudaSuccess)
             return cuda_fail(ctx, e, "cudaMemcpy(shading)");
@@ -340,10 +356,8 @@ extern "C" int32_t ilm_surface_interactions(ilm_context* ctx, ilm_accel_id accel
         return ILM_ERR_INVALID_ARGUMENT;
     }
     const ShadingData& sd = acc->shading;
-    ShadeArgs sa{static_cast<const float4*>(sd.vtx.ptr), static_cast<const float4*>(sd.nrm.ptr),
-                 static_cast<const float4*>(sd.tan.ptr), static_cast<const float2*>(sd.uv.ptr),
-                 static_cast<const uint4*>(sd.tri.ptr),  static_cast<const uint32_t*>(sd.mesh.ptr),
-                 acc->host.n_prims};
+    ShadeArgs sa{static_cast<const float4*>(sd.vtx.ptr), static_cast<const float4*>(sd.tan.ptr),
+                 static_cast<const uint4*>(sd.tri.ptr), acc->host.n_prims};
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
     cudaError_t e;
     if (kr == PtrKind::kDevice) {

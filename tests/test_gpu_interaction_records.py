@@ -52,3 +52,26 @@ def test_records_match_the_oracle(ctx, n, words):
         assert si["kind"][i] == _lib.SI_TRIANGLE
         for f in FIELDS:
             assert np.array_equal(si[f][i], want[f]), (i, f, si[f][i], want[f])
+
+
+def test_meshes_with_and_without_attributes(ctx):
+    """One accel of meshes with all attributes, some and none: every combination in one vertex table."""
+    xyz, idx, rays, extra = scene(23, True)
+    kinds = [{}, extra, {"n": extra["n"]}, {"uv": extra["uv"], "s": extra["s"]}]
+    shift = [np.float32([k, 0, 0]) for k in range(len(kinds))]
+    acc = rb.GpuBVHAccel(ctx, [rb.TriangleMesh(ctx, xyz + d, idx, **kw) for d, kw in zip(shift, kinds)], width=8)
+    rays = np.concatenate([rays] * len(kinds))
+    for k, d in enumerate(shift):
+        rays["o"][k * len(rays) // len(kinds): (k + 1) * len(rays) // len(kinds)] += d
+    hits = acc.intersect_batch(rays)
+    si = acc.surface_interactions(rays, hits)
+    picked = np.random.default_rng(3).permutation(np.nonzero(hits["prim"] != rb.ILM_MISS)[0])[:1200]
+    seen = set()
+    for i in picked:
+        mesh, prim = divmod(int(hits["prim"][i]), len(idx))
+        seen.add(mesh)
+        want = oracle_record(xyz + shift[mesh], idx, prim, rays[i], kinds[mesh])
+        assert si["kind"][i] == _lib.SI_TRIANGLE
+        for f in FIELDS:
+            assert np.array_equal(si[f][i], want[f]), (i, mesh, f, si[f][i], want[f])
+    assert seen == {0, 1, 2, 3}
