@@ -22,7 +22,7 @@
 //
 // Schedules: one thread per ray (grid), or persistent warps that claim rays in
 // chunks and refill finished lanes (the wide BVH kernels' scheme); every loop
-// iteration advances a lane by one node or one leaf.  The pooled persistent
+// iteration advances a lane by up to kKdNodes nodes and a leaf.  The pooled persistent
 // kernel also splits its tail as the wide one does: once every ray is claimed,
 // idle lanes take the top deferred entry of their warp's unfinished rays with
 // its range (KdTracer::give / take).
@@ -52,6 +52,16 @@ __device__ __forceinline__ float pick(uint32_t axis, float x, float y, float z) 
 }
 
 constexpr int kKdBlock = 128;
+
+// Nodes that one pass of a warp takes at most.  A node is about 25 instructions
+// and most passes meet one; with one node a pass, the schedule's ballots and
+// the leaves' triangle tests, which other lanes wait for, came between every
+// two of them, at 14 lanes active.  500,001 ball rays on 327,680 triangles us,
+// closest / any hit, at 1, 3, 5, 6, 8, 10 nodes: 395 / 295, 365 / 227,
+// 286 / 219, 283 / 219, 287 / 222, 298 / 237 (406 / 293 with one node or one
+// leaf a pass); beyond 8 the lanes that have reached a leaf wait too long.
+// Fewer, larger passes leave each ray's own steps and their order as they are.
+constexpr int kKdNodes = 6;
 
 template <bool kAny, bool kAnalytic>
 struct KdTracer {
@@ -87,13 +97,17 @@ struct KdTracer {
         return in;
     }
 
-    // One node or one leaf; true when the ray is finished.
+    // Up to kKdNodes nodes and, where one of them is a leaf, its primitives;
+    // true when the ray is finished.
     __device__ __forceinline__ bool step(const TraceArgs& a) {
-        if ((kAny ? ray.tmax : best_t) < t_min) return true;
-        if (++iter > a.max_iter) { status = kErrIterationCap; return true; }
-        const uint2 nd = __ldg(static_cast<const uint2*>(a.nodes) + cur);
-        const uint32_t axis = nd.y & 3u;
-        if (axis != kKdLeaf) {
+        uint2 nd;
+#pragma unroll 1
+        for (int k = 0;; ++k) {
+            if ((kAny ? ray.tmax : best_t) < t_min) return true;
+            if (++iter > a.max_iter) { status = kErrIterationCap; return true; }
+            nd = __ldg(static_cast<const uint2*>(a.nodes) + cur);
+            const uint32_t axis = nd.y & 3u;
+            if (axis == kKdLeaf) break;
             const float split = __uint_as_float(nd.x);
             const float o = pick(axis, ray.ox, ray.oy, ray.oz);
             const float d = pick(axis, ray.dx, ray.dy, ray.dz);
@@ -112,7 +126,7 @@ struct KdTracer {
                 cur = first;
                 t_max = t_plane;
             }
-            return false;
+            if (k == kKdNodes - 1) return false;
         }
         const uint32_t n = nd.y >> 2;
         for (uint32_t k = 0; k < n; ++k) {
@@ -346,9 +360,10 @@ template <bool kAnalytic>
 cudaError_t launch_kd(const TraceArgs& t, const LaunchParams& lp, cudaStream_t s) {
     if (lp.persistent && t.counter) {
         // Trees of triangles alone always run the build for 8 resident blocks
-        // per SM (62 registers, no spills): 500,001 ball rays on 327,680
-        // triangles 414 against 436 us with the compiler's own
-        // register choice.  With analytic shapes the caller's flag decides.
+        // per SM (64 registers, no spills): 500,001 ball rays on 327,680
+        // triangles 285 against 299 us with the compiler's own register
+        // choice, 262,144 camera rays 357 against 486.  With analytic shapes
+        // the caller's flag decides.
         if constexpr (kAnalytic) {
             if (!lp.high_occupancy)
                 return lp.root_pool ? launch_persistent<1, kAnalytic, true>(t, s)
