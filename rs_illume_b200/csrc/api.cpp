@@ -526,7 +526,7 @@ static int32_t intersect_pageable(ilm_context* ctx, const DeviceAccel& da, Launc
         ILM_CUDA(ctx, st.out.reserve(chunk * sizeof(ilm_hit)), "cudaMalloc(stage out)");
     }
     const size_t slot_bytes = chunk * kRayBytes;   // rays, then results
-    HostCopier& copier = ctx->staging->copier;
+    HostCopier& copier = *ctx->staging->copier;
     cudaStream_t in_s = ctx->pipe[0], out_s = ctx->pipe[1];
     auto count = [&](uint64_t c) { return std::min(chunk, n - c * chunk); };
     auto host_rays = [&](uint64_t c) { return static_cast<char*>(ctx->staging->block) + c % kStageSlots * slot_bytes; };
@@ -642,10 +642,15 @@ static int32_t intersect_impl(ilm_context* ctx, ilm_accel_id accel, const ilm_ra
     if (a->schedule < 0 && da.width != 2 && da.width != kLayoutKdTree) persistent = lp.persistent = 0;
     if (n >= kPageableMin && (pageable(rays) || pageable(out))) {
         if (!ctx->staging) ctx->pageable_rays += std::min(n, kPageableRent);
-        try {
-            if (!ctx->staging && ctx->pageable_rays >= kPageableRent) ctx->staging.reset(new HostStaging());
-            if (ctx->staging && ctx->staging->block)
-                return intersect_pageable(ctx, da, lp, rays, n, hits, occ, err, user);
+        if (!ctx->staging && ctx->pageable_rays >= kPageableRent) {
+            try {
+                ctx->staging.reset(new HostStaging());
+            } catch (const std::bad_alloc&) {
+                // the driver's staging, then
+            }
+        }
+        if (ctx->staging && ctx->staging->block) try {
+            return intersect_pageable(ctx, da, lp, rays, n, hits, occ, err, user);
         } catch (const std::bad_alloc&) {
             cudaDeviceSynchronize();   // no copy may still use the block
             set_error(ctx, "host-buffer query: out of host memory");

@@ -13,9 +13,9 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -23,26 +23,28 @@ namespace ilm {
 
 class HostCopier {
 public:
-    HostCopier() {
+    HostCopier() : s_(new State) {
         const unsigned hw = std::thread::hardware_concurrency();
         const unsigned helpers = hw / 2 < 7 ? hw / 2 : 7;
         try {
-            for (unsigned k = 0; k < helpers; ++k) threads_.emplace_back([this] { helper(); });
-        } catch (const std::system_error&) {
-            // fewer helpers, or none: the caller copies alone
+            s_->threads.reserve(helpers);   // so that a started thread always has its place
+            for (unsigned k = 0; k < helpers; ++k) s_->threads.emplace_back([s = s_] { s->helper(); });
+        } catch (const std::exception&) {
+            // no thread or no memory: fewer helpers, or none: the caller copies alone
         }
     }
     ~HostCopier() {
-        if (getpid() != owner_) {   // a forked child has no helpers to stop or join
-            for (auto& t : threads_) t.detach();
-            return;
-        }
+        // A forked child has no helpers to stop or join, and neither the lock
+        // nor the condition variable that they slept on can be destroyed
+        // there (it would wait for its sleepers): the state stays.
+        if (getpid() != owner_) return;
         {
-            std::lock_guard<std::mutex> lock(mu_);
-            stop_.store(true, std::memory_order_relaxed);
+            std::lock_guard<std::mutex> lock(s_->mu);
+            s_->stop.store(true, std::memory_order_relaxed);
         }
-        wake_.notify_all();
-        for (auto& t : threads_) t.join();
+        s_->wake.notify_all();
+        for (auto& t : s_->threads) t.join();
+        delete s_;
     }
     HostCopier(const HostCopier&) = delete;
     HostCopier& operator=(const HostCopier&) = delete;
@@ -54,13 +56,13 @@ public:
         job->src = static_cast<const char*>(src);
         job->bytes = bytes;
         job->blocks = (bytes + kBlock - 1) / kBlock;
-        if (!threads_.empty() && job->blocks > 1) {
+        if (!s_->threads.empty() && job->blocks > 1) {
             {
-                std::lock_guard<std::mutex> lock(mu_);
-                job_ = job;
-                generation_.fetch_add(1, std::memory_order_relaxed);
+                std::lock_guard<std::mutex> lock(s_->mu);
+                s_->job = job;
+                s_->generation.fetch_add(1, std::memory_order_relaxed);
             }
-            wake_.notify_all();
+            s_->wake.notify_all();
         }
         job->work();
         while (job->done.load(std::memory_order_acquire) != job->blocks) std::this_thread::yield();
@@ -86,52 +88,64 @@ private:
         }
     };
 
-    void helper() {
-        uint64_t seen = 0;
-        for (;;) {
-            for (int k = 0; k < kSpins && generation_.load(std::memory_order_relaxed) == seen &&
-                            !stop_.load(std::memory_order_relaxed);
-                 ++k)
-                pause();
-            std::shared_ptr<Job> job;
-            {
-                std::unique_lock<std::mutex> lock(mu_);
-                wake_.wait(lock, [&] {
-                    return stop_.load(std::memory_order_relaxed) ||
-                           generation_.load(std::memory_order_relaxed) != seen;
-                });
-                if (stop_.load(std::memory_order_relaxed)) return;
-                seen = generation_.load(std::memory_order_relaxed);
-                job = job_;
+    struct State {
+        std::vector<std::thread> threads;
+        std::mutex mu;
+        std::condition_variable wake;
+        std::shared_ptr<Job> job;
+        std::atomic<uint64_t> generation{0};
+        std::atomic<bool> stop{false};
+
+        void helper() {
+            uint64_t seen = 0;
+            for (;;) {
+                for (int k = 0; k < kSpins && generation.load(std::memory_order_relaxed) == seen &&
+                                !stop.load(std::memory_order_relaxed);
+                     ++k)
+                    pause();
+                std::shared_ptr<Job> mine;
+                {
+                    std::unique_lock<std::mutex> lock(mu);
+                    wake.wait(lock, [&] {
+                        return stop.load(std::memory_order_relaxed) ||
+                               generation.load(std::memory_order_relaxed) != seen;
+                    });
+                    if (stop.load(std::memory_order_relaxed)) return;
+                    seen = generation.load(std::memory_order_relaxed);
+                    mine = job;
+                }
+                mine->work();
             }
-            job->work();
         }
-    }
+    };
     static void pause() {
 #if defined(__x86_64__)
         __builtin_ia32_pause();
 #endif
     }
 
+    State* const s_;
     const pid_t owner_ = getpid();
-    std::vector<std::thread> threads_;
-    std::mutex mu_;
-    std::condition_variable wake_;
-    std::shared_ptr<Job> job_;
-    std::atomic<uint64_t> generation_{0};
-    std::atomic<bool> stop_{false};
 };
 
-// One context's staging.  `block` is null if the memory could not be pinned.
+// One context's staging.  If the memory cannot be pinned, `block` and `copier`
+// are null.
 struct HostStaging {
     static constexpr size_t kBlockBytes = 8ull << 20;
+    std::unique_ptr<HostCopier> copier;
     void* block = nullptr;
-    HostCopier copier;
 
     HostStaging() {
         if (cudaHostAlloc(&block, kBlockBytes, cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError();
             block = nullptr;
+            return;
+        }
+        try {
+            copier.reset(new HostCopier());
+        } catch (...) {
+            cudaFreeHost(block);
+            throw;
         }
     }
     ~HostStaging() {
