@@ -58,7 +58,11 @@ struct TraceArgs {
     uint32_t counter_ready = 0;        // LaunchParams::counter_ready
     uint32_t warp_rays = 32;           // k_trace_wide_split: rays a warp starts with, a power of two up to
                                        // 32
+    uint64_t unused = 0;               // see below
 };
+// A launch with 144 bytes of arguments takes 0.35 us longer to enqueue than one
+// with 152 (a one-ray query from C 4.2 against 3.85 us, all of it the host's).
+static_assert(sizeof(TraceArgs) != 144, "pad the arguments");
 
 // occ == nullptr: closest hit into `hits`; otherwise any-hit into `occ`.
 // When n_dev is non-null the kernels trace min(*n_dev, n) rays.
