@@ -37,18 +37,33 @@ __global__ void __launch_bounds__(128) k_trace_wide(TraceArgs a) {
     T.write(i, a);
 }
 
-// Rays a warp of k_trace_wide_split starts with, for n rays on a launch of
-// `threads` resident threads: the smallest power of two (at most 32) whose
-// warps are all resident at once.  The other lanes start idle and take
+// Rays a warp starts with where each ray has a lane of its own, for n rays on a
+// launch of `threads` resident threads.  The other lanes start idle and take
 // subtrees of the warp's rays, so fewer rays a warp shorten the longest ray's
-// chain of steps as long as the warps fit; beyond one wave they queue.
-// Measured us at 32 / 16 / chosen, camera rays on a 32,768-triangle soup:
-// 1,000 rays 84 / 59 / 31 (1 a warp), 10,000 104 / 70 / 43 (4), 33,000
-// 109 / 80 / 76 (8), and at a quarter of the chosen number 62 (10,000) and 98
-// (33,000); incoherent rays gain 0 to 30 %.
-__host__ __device__ __forceinline__ uint32_t rays_per_warp(uint64_t n, uint64_t threads) {
+// chain of steps; but more warps share the SMs' issue slots, and helpers
+// traverse some of what the lone ray would have culled, which weighs more the
+// more rays there are.
+// A path queue takes the smallest power of two (at most 32) whose warps are all
+// resident at once: its rays are coherent, and nearly all enter the scene.
+__host__ __device__ __forceinline__ uint32_t queue_rays_per_warp(uint64_t n, uint64_t threads) {
     uint32_t r = 1;
     while (r < 32u && n * 32u > threads * r) r *= 2u;
+    return r;
+}
+// A query takes r rays a warp while they need at most (16 - r) / 16 of the
+// wave's warps: 1 up to 3,885 rays on 148 SMs of 7 blocks, 2 up to 7,252, 4 up
+// to 12,432, 8 up to 16,576, then 16, and 32 where 16 would not all be resident
+// (66,304).  Against 16 a warp (closest hit, six scenes, camera and incoherent
+// rays): 32 rays 1.36 times as fast, 1,000 1.42, 8,000 1.24, 16,000 1.09.
+// Where 8 a warp would still fit, 20,000 to 33,000 rays, camera rays gain 1.1
+// by it but incoherent ones lose up to 15 %.  us at 32 / 16 / chosen, camera
+// rays on a 32,768-triangle soup: 1,000 rays 84 / 59 / 31, 8,000 101 / 66 / 40,
+// 16,000 107 / 70 / 54.
+inline uint32_t rays_per_warp(uint64_t n, uint64_t threads) {
+    const uint64_t warps = threads / 32u;
+    if (n > 16u * warps) return 32u;
+    uint32_t r = 1;
+    while (r < 16u && 16u * n > warps * r * (16u - r)) r *= 2u;
     return r;
 }
 
@@ -278,7 +293,7 @@ __global__ void __launch_bounds__(128, 7) k_trace_wide_queue(TraceArgs a) {
     __shared__ __align__(16) uint32_t s_warp[4][kWarpWords];
     uint32_t* warp_words = s_warp[threadIdx.x >> 5];
     const uint64_t n = ray_count(a), threads = (uint64_t)gridDim.x * blockDim.x;
-    if (n <= threads) trace_split<W, kStack, kAny, false>(a, n, rays_per_warp(n, threads), warp_words);
+    if (n <= threads) trace_split<W, kStack, kAny, false>(a, n, queue_rays_per_warp(n, threads), warp_words);
     else trace_pooled<W, kStack, kAny, false>(a, n, warp_words);
 }
 
