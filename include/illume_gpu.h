@@ -102,10 +102,12 @@ typedef struct {
  * (warps claim rays in chunks from a per-stream device counter and refill
  * finished lanes). */
 #define ILM_FLAG_GRID_SCHEDULE 2
-/* Persistent schedule compiled for many resident blocks per SM (7 for the
- * wide layouts, up to 72 registers per thread; 8 for kd-trees, 64) instead of
- * the compiler's register choice.  Accels of triangles alone run that build
- * with or without the flag; it decides for accels with quadrics or curves. */
+/* Persistent schedule compiled for many resident blocks per SM instead of the
+ * compiler's register choice: 7 blocks for the wide layouts (up to 72 registers
+ * per thread; 8 and 64 with ILM_FLAG_LANE_REFILL), 8 for kd-trees (64).  Without
+ * the flag, accels of triangles alone run that build where it is the faster
+ * one: kd-trees always, wide layouts in queries of six rays per thread that it
+ * holds resident (795,648 rays on 148 SMs; three with ILM_FLAG_LANE_REFILL). */
 #define ILM_FLAG_HIGH_OCCUPANCY 4
 /* Persistent schedule: each idle lane tests its own claimed rays against the
  * scene's root box instead of the whole warp testing each claimed chunk and
@@ -361,7 +363,7 @@ int32_t ilm_intersect_batched(ilm_context* ctx, const ilm_batch_desc* batches, u
 typedef struct {
     int32_t stack_depth;     /* 32 or 64 */
     int32_t schedule;        /* 0 persistent, 1 one thread per ray */
-    int32_t high_occupancy;  /* 1: 8 resident blocks per SM (64 registers) */
+    int32_t high_occupancy;  /* 1: as ILM_FLAG_HIGH_OCCUPANCY */
 } ilm_launch_opts;
 /* Overrides the context's launch choices for queries on `accel`. */
 int32_t ilm_accel_set_launch(ilm_context* ctx, ilm_accel_id accel, const ilm_launch_opts* opts);

@@ -26,8 +26,9 @@ struct LaunchParams {
     uint32_t max_iter;         // per-ray loop cap
     int persistent;            // wide layouts: persistent schedule (needs `counter`)
     unsigned long long* counter;   // device work counter, private to the launch's stream
-    int high_occupancy;        // persistent kernels with analytic shapes: the build for many resident
-                               // blocks per SM (accels of triangles alone always run it)
+    int high_occupancy;        // persistent kernels: the build for many resident blocks per SM (without
+                               // it, trees of triangles alone run it by wide_deep_query; kd-trees of
+                               // triangles always)
     int root_pool;             // persistent schedule: claimed chunks tested against the root box by the
                                // whole warp, entering rays pooled per warp (1), or each idle lane
                                // testing its own claims (0)
@@ -76,6 +77,9 @@ cudaError_t launch_trace_wide(int width, const TraceArgs& t, const LaunchParams&
 // Rays that one wave of the one-thread-per-ray wide kernel holds resident on
 // the current device (0 when unknown).
 uint64_t wide_grid_wave(int width, int stack_depth);
+// Rays from which a query on triangles alone runs the persistent build for
+// many resident blocks per SM whatever LaunchParams::high_occupancy says.
+uint64_t wide_deep_query(int width, const LaunchParams& lp);
 
 // SMs x resident blocks per SM of `kernel` at `block` threads on the current
 // device (at least one block per SM), cached per (device, kernel) and safe to

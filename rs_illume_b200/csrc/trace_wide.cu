@@ -128,11 +128,11 @@ __global__ void __launch_bounds__(128) k_trace_wide_split(TraceArgs a) {
 // scene, and this keeps the lanes that are still traversing from waiting
 // while a few idle lanes test misses one at a time (5,330 against 4,420
 // Mrays/s on the 2M-ray ball workload).  It carries the split tail.
-template <int W, int kStack, bool kAny, bool kAnalytic>
+template <int W, int kStack, bool kAny, bool kAnalytic, bool kShortClaims>
 __device__ __forceinline__ void trace_pooled(const TraceArgs& a, const uint64_t n, uint32_t* warp_words) {
     // A short queue (fewer than two rays per resident lane) is claimed one ray
     // per lane, so that its rays run side by side rather than two per lane.
-    const unsigned chunk = n < 2ull * gridDim.x * blockDim.x ? 32u : kChunk;
+    const unsigned chunk = kShortClaims || n < 2ull * gridDim.x * blockDim.x ? 32u : kChunk;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned below = (1u << lane) - 1u;
     using Tracer = WideTracer<W, kStack, kAny, kAnalytic>;
@@ -270,13 +270,14 @@ __device__ __forceinline__ void trace_lanes(const TraceArgs& a, const uint64_t n
     }
 }
 
-// kMinBlocks > 0 asks the compiler for that many resident 128-thread blocks
+// kMinBlocks asks the compiler for that many resident 128-thread blocks
 // per SM (launch_refill).
 template <int W, int kStack, bool kAny, int kMinBlocks, bool kAnalytic, bool kPool>
 __global__ void __launch_bounds__(128, kMinBlocks) k_trace_wide_persistent(TraceArgs a) {
     if constexpr (kPool) {
         __shared__ __align__(16) uint32_t s_warp[4][kWarpWords];
-        trace_pooled<W, kStack, kAny, kAnalytic>(a, ray_count(a), s_warp[threadIdx.x >> 5]);
+        trace_pooled<W, kStack, kAny, kAnalytic, W == 8 && kMinBlocks == 1 && !kAnalytic>(
+            a, ray_count(a), s_warp[threadIdx.x >> 5]);
     } else {
         trace_lanes<W, kStack, kAny, kAnalytic>(a, ray_count(a));
     }
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(128, 7) k_trace_wide_queue(TraceArgs a) {
     uint32_t* warp_words = s_warp[threadIdx.x >> 5];
     const uint64_t n = ray_count(a), threads = (uint64_t)gridDim.x * blockDim.x;
     if (n <= threads) trace_split<W, kStack, kAny, false>(a, n, queue_rays_per_warp(n, threads), warp_words);
-    else trace_pooled<W, kStack, kAny, false>(a, n, warp_words);
+    else trace_pooled<W, kStack, kAny, false, false>(a, n, warp_words);
 }
 
 template <int W, int kStack, int kMinBlocks, bool kAnalytic, bool kPool>
@@ -315,22 +316,37 @@ cudaError_t launch_persistent(const TraceArgs& t, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// Persistent launch of either refill.  Accels of triangles alone always run
-// the kernel built for kOccupancyBlocks resident blocks per SM: its state fits
-// 72 registers without spills, and left to itself the compiler takes 80 to 90
-// (5 blocks): 2,000,003 shadow rays on 1.3M triangles 189 against 227 us.
-// With analytic shapes in the leaf loop that build spills 200 to 250 bytes,
-// and the caller's flag decides.
-constexpr int kOccupancyBlocks = 7;
+// Persistent launch of either refill: by the build for many resident blocks
+// per SM (the pooled kernel at 7, whose split tail's state fits 72 registers;
+// the lane-refill kernel at 8, 64 registers, 1 to 9 % faster than at 7) or with
+// the compiler's registers (triangles alone 112 to 122 at width 8, four blocks,
+// and 72 to 90 at width 4; with analytic shapes 112 to 128, where the other
+// build spills up to 242 bytes).  The caller's flag asks for the first; without
+// it, a query on triangles alone takes it from six rays per thread of its wave
+// on (795,648 rays on 148 SMs), lane refill from three.  Long queries have
+// latency to hide all the time: 2,000,000 rays on triangles 1.14 times as fast
+// (closest hit and any hit, six scenes, camera and incoherent rays), 1,000,000
+// 1.06.  In short ones more of the launch is its longest rays, and those run
+// faster with fewer warps beside them: 500,000 incoherent rays on 327,680
+// triangles 104 us against 117, 130,000 64 against 71, and at 700,000 one query
+// in three is still slower.  There the width-8 kernel with the compiler's
+// registers claims 32 rays at a time, one a lane: with 64, 200,000 camera rays
+// took 152 us (140 now), since its 2,368 warps claim 1.3 times each.
+constexpr int kPooledBlocks = 7, kLaneBlocks = 8;
+template <int W, int kStack>
+uint64_t deep_query(bool pooled) {
+    const uint64_t threads =
+        128u * resident_blocks((const void*)k_trace_wide_persistent<W, kStack, false, kPooledBlocks, false, true>, 128);
+    return (pooled ? 6u : 3u) * threads;
+}
+
 template <int W, int kStack, bool kAnalytic>
 cudaError_t launch_refill(const TraceArgs& t, const LaunchParams& lp, cudaStream_t s) {
-    if constexpr (kAnalytic) {
-        if (!lp.high_occupancy)
-            return lp.root_pool ? launch_persistent<W, kStack, 1, kAnalytic, true>(t, s)
-                                : launch_persistent<W, kStack, 1, kAnalytic, false>(t, s);
-    }
-    return lp.root_pool ? launch_persistent<W, kStack, kOccupancyBlocks, kAnalytic, true>(t, s)
-                        : launch_persistent<W, kStack, kOccupancyBlocks, kAnalytic, false>(t, s);
+    if (lp.high_occupancy || (!kAnalytic && t.n >= deep_query<W, kStack>(lp.root_pool != 0)))
+        return lp.root_pool ? launch_persistent<W, kStack, kPooledBlocks, kAnalytic, true>(t, s)
+                            : launch_persistent<W, kStack, kLaneBlocks, kAnalytic, false>(t, s);
+    return lp.root_pool ? launch_persistent<W, kStack, 1, kAnalytic, true>(t, s)
+                        : launch_persistent<W, kStack, 1, kAnalytic, false>(t, s);
 }
 
 template <int W, int kStack, bool kAnalytic>
@@ -388,6 +404,12 @@ uint64_t wide_grid_wave(int width, int stack_depth) {
     const void* k = w8 ? (deep ? (const void*)k_trace_wide<8, 64, false, true> : (const void*)k_trace_wide<8, 32, false, true>)
                        : (deep ? (const void*)k_trace_wide<4, 64, false, true> : (const void*)k_trace_wide<4, 32, false, true>);
     return resident_blocks(k, 128) * 128u;
+}
+
+uint64_t wide_deep_query(int width, const LaunchParams& lp) {
+    const bool deep = lp.stack_depth > 32, pooled = lp.root_pool != 0;
+    return width == 8 ? (deep ? deep_query<8, 64>(pooled) : deep_query<8, 32>(pooled))
+                      : (deep ? deep_query<4, 64>(pooled) : deep_query<4, 32>(pooled));
 }
 
 cudaError_t launch_trace_wide(int width, const TraceArgs& t, const LaunchParams& lp, cudaStream_t s) {
