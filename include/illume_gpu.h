@@ -167,7 +167,7 @@ const char* ilm_last_error_string(const ilm_context* ctx);
  * staging: copy-in and copy-out run on their own streams (the host link
  * carries both directions at once) and a ring of four slots traces on four
  * streams; the first and last chunks ramp from chunk/8.  4096 .. 2^24,
- * default 524288.  Once 2^21 rays have come from pageable buffers in queries
+ * default 524288.  Once 2^19 rays have come from pageable buffers in queries
  * of 8192 rays or more, the context keeps 8 MB of pinned memory and up to seven
  * copying threads (idle between calls) for such queries, whose chunks are then
  * at most 43690 rays; both go with the context. */

@@ -493,10 +493,12 @@ int32_t ilm_accel_binary_nodes(ilm_context* ctx, ilm_accel_id accel, void* out_n
 // the waking of the helpers is most of what there is to save.
 constexpr uint64_t kPageableMin = 8192;
 // The staging is made once this many rays have come in such queries: making it
-// (8 MB to pin, seven threads to start) takes 3 to 10 ms, and by then the
-// driver's way has cost about as much more than it.  A context that makes a
-// few queries never pays for it.
-constexpr uint64_t kPageableRent = 2ull << 20;
+// (8 MB to pin, seven threads to start) adds about 1.1 ms to the query that does,
+// and by then the driver's way has cost about as much more than it.  A context
+// that makes a query or two never pays for it.  Queries of 262,144 rays in a new
+// context: 3.8 ms (the device's staging buffers), 2.2, then 0.5; through the
+// driver throughout 3.8, 1.3, then 1.1.
+constexpr uint64_t kPageableRent = 1ull << 19;
 
 static bool pageable(const void* p) {
     cudaPointerAttributes attr;

@@ -25,14 +25,12 @@ PROGRAM = r"""
 
 static bool pin_fails = false;
 static int pinned = 0;
-extern "C" cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+extern "C" cudaError_t cudaHostRegister(void*, size_t, unsigned) {
     if (pin_fails) return cudaErrorMemoryAllocation;
-    *p = std::malloc(n);
     ++pinned;
     return cudaSuccess;
 }
-extern "C" cudaError_t cudaFreeHost(void* p) {
-    std::free(p);
+extern "C" cudaError_t cudaHostUnregister(void*) {
     --pinned;
     return cudaSuccess;
 }
@@ -81,20 +79,22 @@ int main(int, char** argv) {
         return 0;
     }
     if (what == "fork") {
-        auto* c = new ilm::HostCopier();
+        auto* s = new ilm::HostStaging();
+        ilm::HostCopier* c = s->copier.get();
+        std::memset(s->block, 7, ilm::HostStaging::kBlockBytes);
         if (!copies(*c)) return 1;
         std::this_thread::sleep_for(std::chrono::milliseconds(200));   // the helpers sleep
         const pid_t child = fork();
         if (child == 0) {
             alarm(10);
-            delete c;
-            _exit(0);
+            delete s;
+            _exit(pinned == 1 ? 0 : 1);   // the parent's
         }
         int status = -1;
         waitpid(child, &status, 0);
-        const bool ok = copies(*c);    // the parent's are as they were
-        delete c;
-        return status == 0 && ok ? 0 : 1;
+        const bool ok = copies(*c) && static_cast<char*>(s->block)[ilm::HostStaging::kBlockBytes - 1] == 7;
+        delete s;
+        return status == 0 && ok && pinned == 0 ? 0 : 1;
     }
     if (what == "no_memory") {
         int made = 0;
