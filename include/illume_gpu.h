@@ -373,7 +373,7 @@ typedef struct {
     ilm_launch_opts launch;  /* best launch choices at that width */
     double ms;               /* its median time on the sample */
     double baseline_ms;      /* width 8, context defaults, same sample */
-    uint32_t n_tried;
+    uint32_t n_tried;        /* launch choices considered (two that run the same kernel are timed once) */
     int32_t from_cache;      /* 1 when answered from the context's cache */
 } ilm_tune_result;
 /* Builds the shapes' accel at widths 2, 4 and 8, times every launch choice on

@@ -115,7 +115,16 @@ int32_t ilm_autotune(ilm_context* ctx, const ilm_mesh_id* meshes, uint32_t n_mes
                 choices.push_back({sd, 0, 1});
                 choices.push_back({sd, 1, 0});
             }
+        // Large samples on triangles alone run the many-blocks build with or
+        // without the flag: the choice before it has its time already.
+        const Accel* built = find_accel(ctx, acc);
+        const bool flag_idle = width != 2 && !built->view().spheres &&
+                               n >= wide_deep_query(width, accel_launch(ctx, built));
         for (const ilm_launch_opts& c : choices) {
+            if (c.high_occupancy && flag_idle) {
+                ++tried;
+                continue;
+            }
             if (width != 2) ilm_accel_set_launch(ctx, acc, &c);
             double ms = 0.0;
             if ((status = time_it(acc, &ms)) != ILM_OK) break;
