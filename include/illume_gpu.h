@@ -476,7 +476,9 @@ int32_t ilm_nrc_destroy(ilm_context* ctx, ilm_nrc* nrc);
 /* Reads (get) and/or replaces (set) the FP32 master weights, row-major
  * [out][in] per layer, layers in order. */
 int32_t ilm_nrc_params(ilm_context* ctx, ilm_nrc* nrc, float* get, const float* set);
-/* out[n][3] = network(inputs[n][12]); host or device buffers. */
+/* out[n][3] = network(inputs[n][12]); host or device buffers.  The encoding rounds
+ * rows 128 apart differently: about one row in 7,000 gets answers a bf16 rounding
+ * apart at another place of a batch. */
 int32_t ilm_nrc_infer(ilm_context* ctx, ilm_nrc* nrc, const float* inputs, uint64_t n, float* out, void* stream);
 /* One Adam step on the batch; *loss (optional) receives the batch loss. */
 int32_t ilm_nrc_train_step(ilm_context* ctx, ilm_nrc* nrc, const float* inputs, const float* targets,

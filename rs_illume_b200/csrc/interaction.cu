@@ -236,7 +236,7 @@ __device__ __forceinline__ void surface_interaction(const ShadeArgs& sa, const i
 // triangle, mesh flags and positions, then normals and uvs) with 20 warps an SM
 // to hide it: vertices of one sector each, read at once, 67 us; the words of a
 // record written as they are known, which frees the registers of three more
-// blocks, 53 us (8 blocks; 55 at 7, 68 at 9, which spill), 4,430 GB/s of the 48
+// blocks, 53 us (8 blocks, which spill 24 bytes; 55 at 7, 68 at 9), 4,430 GB/s of the 48
 // and 176 bytes.  kAligned: rays, hits and out on 16-byte boundaries (every
 // buffer a query accepts is; this entry point also takes 4-byte aligned ones,
 // which are read and written word by word, the writes still coalesced).

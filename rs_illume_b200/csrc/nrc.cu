@@ -330,8 +330,13 @@ __device__ __forceinline__ void load_raw(const float* __restrict__ raw, uint32_t
 // (s, c) (octave 0: from q); (s, c) becomes the last one.  The doubling is
 // feature_group's, each operation rounded by itself, except that c - s and
 // c + s of octave kFuse round once with the product that s is (kFuse < 0:
-// none).  Which octaves those are is what the compiler made of this kernel's
-// two-tile form; it is kept so that its answers stay the same to the last bit.
+// none).  Which octaves those are is the rounding that this kernel has had since
+// it worked on tiles in pairs, and it differs between even and odd tiles: about
+// one row in 7,000 gets answers a bf16 rounding apart in the two (4e-5 to 6e-5
+// of the answers' norm in all).  It is kept because one rule for all tiles, which
+// is no nearer to 64 bits (0.0072 either way), changes answers by as much
+// (4.5e-5).  The training kernel and k_nrc_encode round every row by
+// feature_group.
 template <int O0, int kFuse>
 __device__ __forceinline__ void octaves(float q, float& s, float& c, uint32_t (&w)[4]) {
     float s1 = s, c1 = c;   // the octave before (s, c)

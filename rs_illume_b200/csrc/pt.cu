@@ -298,10 +298,10 @@ __global__ void k_pt_camera(PtArgs a, unsigned long long p0, uint32_t count) {
 // holding all of them to the end took 124 to 162 registers (two blocks per
 // SM).  The stage streams about 140 bytes a path in and 50 to 150 out, but is
 // bound by issue and the latency of hit -> triangle -> material -> light, so
-// three blocks per SM pay for the 50 to 100 bytes they spill: shading of a
-// 1024 x 1024 render at 16 spp 5.17 ms before, 4.35 now (4.65 at four blocks),
-// of four cache frames 1.39 and 0.82.  (Appending once per block instead made
-// the queues' order cost the traversal 0.6 ms of the render.)
+// three blocks per SM pay for the bytes they spill (52, with the cache 124):
+// shading of a 1024 x 1024 render at 16 spp 5.17 ms before, 4.35 now (4.65 at
+// four blocks), of four cache frames 1.39 and 0.82.  (Appending once per block
+// instead made the queues' order cost the traversal 0.6 ms of the render.)
 constexpr int kShadeBlock = 256;
 template <bool kNrc>
 __global__ void __launch_bounds__(kShadeBlock, 3) k_pt_shade(PtArgs a, int cur) {

@@ -60,7 +60,8 @@ constexpr int kKdBlock = 128;
 // closest / any hit, at 1, 3, 5, 6, 8, 10 nodes: 395 / 295, 365 / 227,
 // 286 / 219, 283 / 219, 287 / 222, 298 / 237 (406 / 293 with one node or one
 // leaf a pass); beyond 8 the lanes that have reached a leaf wait too long.
-// Fewer, larger passes leave each ray's own steps and their order as they are.
+// Fewer, larger passes leave a ray's own steps and their order as they are; in
+// the split tail they decide which lane takes which deferred entry.
 constexpr int kKdNodes = 6;
 
 template <bool kAny, bool kAnalytic>
@@ -360,10 +361,11 @@ template <bool kAnalytic>
 cudaError_t launch_kd(const TraceArgs& t, const LaunchParams& lp, cudaStream_t s) {
     if (lp.persistent && t.counter) {
         // Trees of triangles alone always run the build for 8 resident blocks
-        // per SM (64 registers, no spills): 500,001 ball rays on 327,680
-        // triangles 285 against 299 us with the compiler's own register
-        // choice, 262,144 camera rays 357 against 486.  With analytic shapes
-        // the caller's flag decides.
+        // per SM (64 registers; closest hit spills 8 bytes pooled and 40 with
+        // lane refill, any hit none): 500,001 ball rays on 327,680 triangles
+        // 285 against 299 us with the compiler's own register choice, 262,144
+        // camera rays 357 against 486.  With analytic shapes the caller's flag
+        // decides.
         if constexpr (kAnalytic) {
             if (!lp.high_occupancy)
                 return lp.root_pool ? launch_persistent<1, kAnalytic, true>(t, s)
